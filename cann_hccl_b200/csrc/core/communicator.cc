@@ -631,6 +631,7 @@ HcclResult Communicator::collective(const OpRequest &rq)
     }
     HcclResult ready = check_ready();
     const bool dev = settings_.transport == TR_DEVICE;
+    const bool can_retry_ops = dev && !all_local_ && nranks_ > 1;  // ranks in other processes whose kernels may fail after the call
     const bool can_retry = env_config().retry_enable && !all_local_ && nranks_ > 1 && (ready == HCCL_E_TIMEOUT || ready == HCCL_E_REMOTE);
     bool own_fail = false;
     for (auto *st : status_) own_fail = own_fail || (st && st->code != 0);
@@ -653,7 +654,7 @@ HcclResult Communicator::collective(const OpRequest &rq)
     StateGuard guard(state_, CS_INUSE);
     const bool nvtx = env_config().nvtx;
     if (nvtx) nvtxRangePushA(coll_name(rq.coll));
-    if (dev && !calibrating_) remember_op(rq);
+    if (can_retry_ops && !calibrating_) remember_op(rq);
     HcclResult rc = peer_failed ? ready : run_collective_once(rq);
     if (rc != HCCL_SUCCESS && (rc == HCCL_E_TIMEOUT || rc == HCCL_E_REMOTE)) {
         stats_.timeouts++;
@@ -687,6 +688,20 @@ HcclResult Communicator::run_collective_once(const OpRequest &rq)
         for (int j = 0; j < p; ++j) sel_count += rq.send_counts[j];
     }
     if (is_v) sel_count = window;
+    if (direct_applies(rq)) {
+        if (is_a2av) CHK_RET(a2av_check(rq));
+        int h0 = 0;
+        size_t o0 = 0;
+        const int label = p == 1 ? ALGO_SINGLE : (zc_candidate(rq) && registered_send(rq, &h0, &o0) ? ALGO_MESH_ZC : ALGO_DIRECT);
+        ++direct_ops_;
+        for (int li = 0; li < nl; ++li) __atomic_store_n(&status_[li]->head, direct_ops_, __ATOMIC_RELAXED);
+        HcclResult drc = run_direct(rq);
+        stats_.ops[rq.coll]++;
+        stats_.bytes[rq.coll] += sel_count * es;
+        stats_.algo_hist[label]++;
+        record_trace(rq, label, 0, sel_count * es, now_us() - t0);
+        return drc;
+    }
     Selection sel = select(rq.coll, sel_count, rq.dtype, rq.redop);
     if (rq.algo != ALGO_AUTO) sel.algo = rq.algo;
     if (rq.nchan > 0) sel.nchan = rq.nchan;
@@ -752,22 +767,10 @@ HcclResult Communicator::run_collective_once(const OpRequest &rq)
 
     // registered send buffer (the same allocation and offset on every rank, by the contract of symmetric memory): two-rank
     // AllReduce, ReduceScatter and AllGather let the peers read it where it is
-    if (!use_zc && settings_.transport == TR_DEVICE && p > 1 && !user_segs_.empty() && (rq.algo == ALGO_AUTO || rq.algo == ALGO_MESH_ZC) &&
-        ((rq.coll == COLL_ALLREDUCE && p == 2) || rq.coll == COLL_REDUCE_SCATTER || rq.coll == COLL_ALLGATHER) &&
-        (rq.algo == ALGO_MESH_ZC || rq.count * es >= (1u << 20)) && forced_algo_for(env_config(), rq.coll).empty()) {
-        const size_t in_bytes = (size_t)rq.count * es * (rq.coll == COLL_REDUCE_SCATTER ? p : 1);
+    if (!use_zc && zc_candidate(rq)) {
         int h0 = 0;
         size_t o0 = 0;
-        bool mine = true;
-        for (int li = 0; li < nl && mine; ++li) {
-            size_t o = 0;
-            int h = find_user_seg(li, rq.in[li], in_bytes, &o);
-            if (li == 0) { h0 = h; o0 = o; }
-            mine = h != 0 && h == h0 && o == o0 && (o & 15) == 0;
-            // AllReduce in place would overwrite what the peer is still reading: that form stays on the staged paths
-            if (rq.coll == COLL_ALLREDUCE && overlap_kind(rq, li) != 0) mine = false;
-        }
-        if (mine) {
+        if (registered_send(rq, &h0, &o0)) {
             CHK_RET(consistency_check(rq, ALGO_MESH_ZC, ((uint64_t)h0 << 48) ^ o0, 0));
             HcclResult zrc = run_pipe(rq, false, h0, o0);
             uint64_t zbytes = sel_count * es;
@@ -874,6 +877,29 @@ HcclResult Communicator::run_collective_once(const OpRequest &rq)
     stats_.algo_hist[sel.algo]++;
     record_trace(rq, sel.algo, sel.nchan, bytes, now_us() - t0);
     return rc;
+}
+
+// Collectives, sizes and requests for which a registered send buffer means that the peers read it in place.
+bool Communicator::zc_candidate(const OpRequest &rq) const
+{
+    return settings_.transport == TR_DEVICE && nranks_ > 1 && !user_segs_.empty() && (rq.algo == ALGO_AUTO || rq.algo == ALGO_MESH_ZC) &&
+           ((rq.coll == COLL_ALLREDUCE && nranks_ == 2) || rq.coll == COLL_REDUCE_SCATTER || rq.coll == COLL_ALLGATHER) &&
+           (rq.algo == ALGO_MESH_ZC || rq.count * (uint64_t)dtype_size(rq.dtype) >= (1u << 20)) && forced_algo_for(env_config(), rq.coll).empty();
+}
+
+// The send buffers of all local ranks lie in one registered allocation at one offset.
+bool Communicator::registered_send(const OpRequest &rq, int *handle, size_t *offset)
+{
+    const size_t in_bytes = (size_t)rq.count * dtype_size(rq.dtype) * (rq.coll == COLL_REDUCE_SCATTER ? nranks_ : 1);
+    for (int li = 0; li < nlocal(); ++li) {
+        size_t o = 0;
+        int h = find_user_seg(li, rq.in[li], in_bytes, &o);
+        if (li == 0) { *handle = h; *offset = o; }
+        if (h == 0 || h != *handle || o != *offset || (o & 15) != 0) return false;
+        // AllReduce in place would overwrite what the peer is still reading: that form stays on the staged paths
+        if (rq.coll == COLL_ALLREDUCE && overlap_kind(rq, li) != 0) return false;
+    }
+    return true;
 }
 
 int Communicator::pipe_mode_for(int coll) const

@@ -183,6 +183,10 @@ private:
     HcclResult run_ll_allreduce(const OpRequest &rq);
     HcclResult run_pipe(const OpRequest &rq, bool want_mc, int zc_handle = 0, size_t zc_off = 0);
     HcclResult run_a2av(const OpRequest &rq);
+    bool direct_applies(const OpRequest &rq) const;  // core/direct.cc: all ranks in this process on one GPU
+    HcclResult run_direct(const OpRequest &rq);
+    bool zc_candidate(const OpRequest &rq) const;
+    bool registered_send(const OpRequest &rq, int *handle, size_t *offset);
     int pipe_mode_for(int coll) const;  // PipeMode of a collective, -1 when it has no pipelined kernel
     HcclResult tp_workspace(const std::string &key, size_t data_bytes, int M, void **ws_out);
     void tp_release_workspaces();
@@ -234,6 +238,7 @@ private:
     void *pinned_ = nullptr;               // host-mapped block holding status + abort words
     uint64_t p2p_slot_ = 0;
     uint64_t ll_seq_ = 0;                  // number of LL operations issued (tag and mailbox parity)
+    uint64_t direct_ops_ = 1ull << 62;     // op-execution id of the direct path (it consumes no plan sequence number)
     bool ll_ok_ = false;
     uint64_t ll_two_shot_min_ = 256u << 10;  // from this size on the LL path of three and more ranks goes two-shot
     uint64_t ll_max_bytes() const;            // largest message the LL path takes on this communicator

@@ -1,0 +1,194 @@
+"""Direct collectives of communicators that hold every rank in this process on one GPU (algorithm left to the selector),
+against a plain PyTorch reference: sizes around vectors and tiles, every alignment, in-place forms."""
+import pytest
+
+torch = pytest.importorskip("torch")
+import numpy as np  # noqa: E402
+import cann_hccl_b200 as H  # noqa: E402
+from cann_hccl_b200 import _lib as L  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+# below a vector; around one vector and one tile of 256 threads; around many tiles of the unrolled form
+SIZES = (1, 3, 17, 4095, 4097, 1_300_001)
+
+
+@pytest.fixture(scope="module")
+def comms():
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    cache = {}
+
+    def get(p):
+        if p not in cache:
+            cfg = L.CommConfig.default()
+            cfg.hcclBufferSize = 2
+            cache[p] = H.Communicator.init_local(p, device=True, device_id=0, config=cfg)
+        return cache[p]
+
+    yield get
+    for c in cache.values():
+        assert c.destroy() == L.SUCCESS
+
+
+def rnd(p, n, dtype, seed, shift=lambda r: 0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    out = []
+    for r in range(p):
+        x = torch.rand(n + 16, device="cuda", generator=g) * 2 - 1
+        x = x.to(dtype) if dtype.is_floating_point else (x * 4).to(dtype)
+        out.append(x[shift(r):shift(r) + n])
+    return out
+
+
+def reduced(ins, op):
+    acc = ins[0].double() if ins[0].dtype.is_floating_point else ins[0].clone()
+    for x in ins[1:]:
+        y = x.to(acc.dtype)
+        acc = {L.SUM: acc + y, L.PROD: acc * y, L.MAX: torch.maximum(acc, y), L.MIN: torch.minimum(acc, y)}[op]
+    return acc
+
+
+def check(got, want, dtype, p):
+    if not dtype.is_floating_point:
+        assert torch.equal(got, want)
+        return
+    # p - 1 roundings of the accumulator (unit roundoff of fp32 / fp64), one of the result, values below p in magnitude
+    eps = {torch.float64: 2.0 ** -52, torch.float32: 2.0 ** -23, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype]
+    assert float((got.double() - want).abs().max()) <= p * p * eps
+
+
+def done(c, algo="direct"):
+    assert c.sync() == 0, c.describe_status()
+    assert c.trace()[-1]["algo"] == algo, c.trace()[-1]
+
+
+@pytest.mark.parametrize("p", [2, 3, 4, 8, 11])
+@pytest.mark.parametrize("dtype,op", [(torch.float32, L.SUM), (torch.bfloat16, L.SUM), (torch.float16, L.MAX), (torch.int8, L.MIN),
+                                      (torch.int64, L.PROD), (torch.float64, L.SUM)])
+def test_reductions(comms, p, dtype, op):
+    c = comms(p)
+    for n in SIZES:
+        ins = rnd(p, n, dtype, n)
+        outs = [torch.full_like(x, 9) for x in ins]
+        c.all_reduce(ins, outs, op=op)
+        done(c)
+        want = reduced(ins, op)
+        for o in outs:
+            check(o, want, dtype, p)
+        outs = [torch.full_like(x, 9) for x in ins]
+        c.reduce(ins, outs, p - 1, op=op)
+        done(c)
+        check(outs[p - 1], want, dtype, p)
+        assert all(bool((o == 9).all()) for o in outs[:-1])     # only the root's buffer is written
+        m = max(1, n // p)
+        ins = rnd(p, m * p, dtype, n + 1)                        # odd blocks start anywhere inside a vector
+        outs = [torch.full((m,), 9, device="cuda", dtype=dtype) for _ in range(p)]
+        c.reduce_scatter(ins, outs, op=op)
+        done(c)
+        want = reduced(ins, op)
+        for r, o in enumerate(outs):
+            check(o, want[r * m:(r + 1) * m], dtype, p)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.uint8])
+@pytest.mark.parametrize("shift_in,shift_out", [(1, 0), (0, 1), (3, 3), (5, 2), (-1, 0), (0, -1)])
+def test_alignments(comms, dtype, shift_in, shift_out):
+    """Every rank's buffers at the same offset from a 16-byte boundary, or (negative) at a different one on each rank."""
+    p, n = 4, 100_003
+    c = comms(p)
+    at = lambda s: (lambda r: s if s >= 0 else r * 3 % 7)
+    ins = rnd(p, n, dtype, 5, at(shift_in))
+    base = [torch.full((n + 32,), 9, device="cuda", dtype=dtype) for _ in range(p)]
+    outs = [b[8 + at(shift_out)(r):8 + at(shift_out)(r) + n] for r, b in enumerate(base)]
+    c.all_reduce(ins, outs, op=L.MAX)
+    done(c)
+    for o in outs:
+        assert torch.equal(o.float(), reduced(ins, L.MAX).float())
+    for r, b in enumerate(base):                                 # nothing around the output was touched
+        lo = 8 + at(shift_out)(r)
+        assert bool((b[:lo] == 9).all()) and bool((b[lo + n:] == 9).all())
+    gbase = [torch.full((n * p + 32,), 9, device="cuda", dtype=dtype) for _ in range(p)]
+    gout = [b[8 + at(shift_out)(r):8 + at(shift_out)(r) + n * p] for r, b in enumerate(gbase)]
+    c.all_gather(ins, gout)
+    done(c)
+    for r, (o, b) in enumerate(zip(gout, gbase)):
+        assert torch.equal(o, torch.cat(ins))
+        lo = 8 + at(shift_out)(r)
+        assert bool((b[:lo] == 9).all()) and bool((b[lo + n * p:] == 9).all())
+
+
+@pytest.mark.parametrize("p", [2, 5])
+def test_in_place(comms, p):
+    c = comms(p)
+    n = 70_001
+    ins = rnd(p, n, torch.float32, 1)
+    want = reduced(ins, L.SUM)
+    c.all_reduce(ins, ins)
+    done(c)
+    for x in ins:
+        check(x, want, torch.float32, p)
+    ins = rnd(p, n * p, torch.float32, 2)
+    want = reduced(ins, L.SUM)
+    c.reduce_scatter(ins, [x[r * n:(r + 1) * n] for r, x in enumerate(ins)])
+    done(c)
+    for r, x in enumerate(ins):
+        check(x[r * n:(r + 1) * n], want[r * n:(r + 1) * n], torch.float32, p)
+    full = rnd(p, n * p, torch.float32, 3)
+    blocks = [x[r * n:(r + 1) * n].clone() for r, x in enumerate(full)]
+    c.all_gather([x[r * n:(r + 1) * n] for r, x in enumerate(full)], full)
+    done(c)
+    for x in full:
+        assert torch.equal(x, torch.cat(blocks))
+
+
+@pytest.mark.parametrize("p", [2, 4, 9])
+def test_copies(comms, p):
+    c = comms(p)
+    for n in SIZES:
+        n = min(n, 100_003)
+        bufs = rnd(p, n, torch.float32, n)
+        want = bufs[p - 1].clone()
+        c.broadcast(bufs, p - 1)
+        done(c)
+        assert all(torch.equal(b, want) for b in bufs)
+        big, small = rnd(p, n * p, torch.bfloat16, n), [torch.zeros(n, device="cuda", dtype=torch.bfloat16) for _ in range(p)]
+        c.scatter(big, small, 1)
+        done(c)
+        assert torch.equal(torch.cat(small), big[1])
+        back = [torch.zeros_like(x) for x in big]
+        c.gather(small, back, 0)
+        done(c)
+        assert torch.equal(back[0], big[1])
+        out = [torch.zeros_like(x) for x in big]
+        c.all_to_all(big, out)
+        done(c)
+        for r in range(p):
+            assert torch.equal(out[r], torch.cat([big[q][r * n:(r + 1) * n] for q in range(p)]))
+
+
+def test_variable_counts(comms):
+    p = 4
+    c = comms(p)
+    counts, displs = np.array([5, 0, 4101, 33], np.uint64), np.array([0, 8, 16, 4200], np.uint64)
+    total = 4300
+    ins = [rnd(1, max(1, int(counts[r])), torch.float32, r)[0] for r in range(p)]
+    outs = [torch.full((total,), 9.0, device="cuda") for _ in range(p)]
+    c.all_gather_v(ins, outs, counts, displs)
+    done(c)
+    want = torch.full((total,), 9.0, device="cuda")
+    for r in range(p):
+        want[int(displs[r]):int(displs[r] + counts[r])] = ins[r][:int(counts[r])]
+    assert all(torch.equal(o, want) for o in outs)
+    rin = rnd(p, total, torch.float32, 9)
+    rout = [torch.full((5000,), 9.0, device="cuda") for _ in range(p)]
+    c.reduce_scatter_v(rin, rout, counts, displs)
+    done(c)
+    ref = reduced(rin, L.SUM)
+    for r in range(p):
+        k = int(counts[r])
+        if k:
+            check(rout[r][:k], ref[int(displs[r]):int(displs[r]) + k], torch.float32, p)
+        assert bool((rout[r][k:] == 9).all())
+    c.barrier()
+    assert c.sync() == 0
