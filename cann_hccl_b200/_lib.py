@@ -1,6 +1,8 @@
 """ctypes binding of libhccl_b200.so (the C API of include/hccl/hccl.h and hccl_b200.h)."""
 import ctypes as C
 import os
+from importlib.machinery import ExtensionFileLoader
+from importlib.util import module_from_spec, spec_from_loader
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
 # HCCL_B200_LIB: another build of the library (a sanitizer build, for one)
@@ -82,6 +84,7 @@ class B200Status(C.Structure):
 
 
 _lib = None
+fast = None  # csrc/python/fastcall.c, bound to the loaded library
 
 
 def _nccl_path():
@@ -98,11 +101,11 @@ def _nccl_path():
 
 def lib():
     """Load (building first when missing) the native library."""
-    global _lib
+    global _lib, fast
     if _lib is not None:
         return _lib
-    if not os.path.exists(LIB_PATH):
-        from . import build as _build
+    from . import build as _build
+    if not os.path.exists(LIB_PATH) or not os.path.exists(_build.fastcall_path()):
         _build.build()
     if "HCCL_NCCL_LIB" not in os.environ:
         p = _nccl_path()
@@ -216,6 +219,10 @@ def lib():
     L.HcclB200AlgoName.restype = C.c_char_p
     L.HcclGetCommConfigCapability.argtypes = []
     L.HcclGetCommConfigCapability.restype = C.c_uint32
+    loader = ExtensionFileLoader("_fastcall", _build.fastcall_path())
+    fast = module_from_spec(spec_from_loader("_fastcall", loader))
+    loader.exec_module(fast)
+    fast.bind(C.cast(L.HcclB200Collective, vp).value)
     _lib = L
     return L
 

@@ -16,6 +16,7 @@ thread sanitizer (objects under build_<kind>/).  Run the CPU suite on it with
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 PKG = os.path.dirname(os.path.abspath(__file__))
@@ -71,6 +72,23 @@ def lib_path(sanitize=None):
     return os.path.join(LIB, "libhccl_b200_%s.so" % sanitize if sanitize else "libhccl_b200.so")
 
 
+def fastcall_path():
+    """The call path of the Python layer (csrc/python/fastcall.c), an extension module of the running interpreter."""
+    return os.path.join(LIB, "_fastcall.so")
+
+
+def _build_fastcall(force, verbose):
+    src, out = os.path.join(CSRC, "python", "fastcall.c"), fastcall_path()
+    if not force and os.path.exists(out) and os.path.getmtime(out) >= max(os.path.getmtime(src), _newest_header()):
+        return
+    cmd = ["gcc", "-O2", "-g", "-fPIC", "-shared", "-std=c11", "-Wall", "-I" + INC, "-I" + sysconfig.get_paths()["include"], src, "-o", out]
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("compile failed: %s\n%s\n%s" % (" ".join(cmd), r.stdout, r.stderr))
+
+
 def build(force=False, verbose=False, sanitize=None):
     global OBJ, CXXFLAGS, NVCCFLAGS
     san_link = []
@@ -84,6 +102,7 @@ def build(force=False, verbose=False, sanitize=None):
         san_link = ["-Xcompiler", flag]
     os.makedirs(OBJ, exist_ok=True)
     os.makedirs(LIB, exist_ok=True)
+    _build_fastcall(force, verbose)
     hdr = _newest_header()
     jobs, objs = [], []
     for src in _sources():

@@ -1,0 +1,118 @@
+/* Call path of the Python layer: one METH_FASTCALL function per C API entry that sits on a latency path.  It takes the tensors
+ * as they are, asks each for its address, fills the argument structure on the stack and calls the library with the
+ * interpreter lock released.  Through ctypes the same call costs several microseconds (argument objects, one pointer array per
+ * buffer list), as much as a small collective takes on the GPU.  No PyTorch headers: addresses come from data_ptr(). */
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+#include <stdint.h>
+#include <string.h>
+#include "hccl/hccl_b200.h"
+
+#define MAX_LOCAL 16
+
+typedef HcclResult (*collective_fn)(HcclComm, const HcclB200Op *, void *const *, void *const *, aclrtStream);
+static collective_fn g_collective;
+static PyObject *s_data_ptr, *s_ctypes, *s_data;
+
+/* address of a tensor (data_ptr()) or numpy array (ctypes.data); None is null */
+static int address(PyObject *x, void **out)
+{
+    if (x == Py_None) { *out = NULL; return 0; }
+    PyObject *v = PyObject_CallMethodNoArgs(x, s_data_ptr);
+    if (!v) {
+        if (!PyErr_ExceptionMatches(PyExc_AttributeError)) return -1;
+        PyErr_Clear();
+        PyObject *c = PyObject_GetAttr(x, s_ctypes);
+        if (!c) return -1;
+        v = PyObject_GetAttr(c, s_data);
+        Py_DECREF(c);
+        if (!v) return -1;
+    }
+    *out = PyLong_AsVoidPtr(v);
+    Py_DECREF(v);
+    return *out == NULL && PyErr_Occurred() ? -1 : 0;
+}
+
+/* one address per local rank; a rank that is alone may pass its buffer without a list */
+static int addresses(PyObject *x, Py_ssize_t nlocal, void **out)
+{
+    const int list = PyList_Check(x), tuple = PyTuple_Check(x);
+    if (!list && !tuple) {
+        if (nlocal == 1) return address(x, out);
+        PyErr_SetString(PyExc_AssertionError, "need one buffer per local rank");
+        return -1;
+    }
+    const Py_ssize_t n = list ? PyList_GET_SIZE(x) : PyTuple_GET_SIZE(x);
+    if (n != nlocal) { PyErr_SetString(PyExc_AssertionError, "need one buffer per local rank"); return -1; }
+    for (Py_ssize_t i = 0; i < n; ++i)
+        if (address(list ? PyList_GET_ITEM(x, i) : PyTuple_GET_ITEM(x, i), out + i)) return -1;
+    return 0;
+}
+
+/* the caller has made these contiguous arrays of 64-bit unsigned integers */
+static int words(PyObject *x, Py_buffer *view, const uint64_t **out)
+{
+    if (PyObject_GetBuffer(x, view, PyBUF_SIMPLE)) return -1;
+    *out = (const uint64_t *)view->buf;
+    return 0;
+}
+
+/* bind(address of HcclB200Collective) */
+static PyObject *bind(PyObject *self, PyObject *const *a, Py_ssize_t n)
+{
+    if (n != 1) { PyErr_SetString(PyExc_TypeError, "bind() takes one address"); return NULL; }
+    g_collective = (collective_fn)PyLong_AsVoidPtr(a[0]);
+    if (PyErr_Occurred()) return NULL;
+    Py_RETURN_NONE;
+}
+
+/* collective(comm, nlocal, coll, algo, nchan, dtype, op, root, count, send, recv, stream, tables) -> result code
+ * tables: None, (counts, displs) or (sendCounts, sdispls, recvCounts, rdispls) */
+static PyObject *collective(PyObject *self, PyObject *const *a, Py_ssize_t n)
+{
+    if (n != 13 || !g_collective) { PyErr_SetString(PyExc_TypeError, "collective() takes 13 arguments, after bind()"); return NULL; }
+    HcclB200Op o;
+    memset(&o, 0, sizeof(o));
+    void *comm = PyLong_AsVoidPtr(a[0]), *stream = a[11] == Py_None ? NULL : PyLong_AsVoidPtr(a[11]);
+    const Py_ssize_t nlocal = PyLong_AsSsize_t(a[1]);
+    o.coll = (int32_t)PyLong_AsLong(a[2]); o.algo = (int32_t)PyLong_AsLong(a[3]); o.nchan = (int32_t)PyLong_AsLong(a[4]);
+    o.dataType = (int32_t)PyLong_AsLong(a[5]); o.op = (int32_t)PyLong_AsLong(a[6]); o.root = (int32_t)PyLong_AsLong(a[7]);
+    o.count = PyLong_AsUnsignedLongLong(a[8]);
+    if (PyErr_Occurred()) return NULL;
+    if (nlocal < 1 || nlocal > MAX_LOCAL) { PyErr_SetString(PyExc_ValueError, "bad number of local ranks"); return NULL; }
+    void *send[MAX_LOCAL], *recv[MAX_LOCAL];
+    const int barrier = o.coll == HCCL_B200_BARRIER;
+    if (!barrier && (addresses(a[9], nlocal, send) || addresses(a[10], nlocal, recv))) return NULL;
+    Py_buffer view[4];
+    int nview = 0;
+    if (a[12] != Py_None) {
+        const uint64_t *w[4] = {NULL, NULL, NULL, NULL};
+        const Py_ssize_t m = PyTuple_GET_SIZE(a[12]);
+        for (; nview < m && nview < 4; ++nview)
+            if (words(PyTuple_GET_ITEM(a[12], nview), &view[nview], &w[nview])) goto fail;
+        if (m == 2) { o.counts = w[0]; o.displs = w[1]; }
+        else { o.sendCounts = w[0]; o.sdispls = w[1]; o.recvCounts = w[2]; o.rdispls = w[3]; }
+    }
+    HcclResult rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = g_collective((HcclComm)comm, &o, barrier ? NULL : send, barrier ? NULL : recv, (aclrtStream)stream);
+    Py_END_ALLOW_THREADS
+    while (nview) PyBuffer_Release(&view[--nview]);
+    return PyLong_FromLong((long)rc);
+fail:
+    while (nview) PyBuffer_Release(&view[--nview]);
+    return NULL;
+}
+
+static PyMethodDef methods[] = {{"bind", (PyCFunction)(void (*)(void))bind, METH_FASTCALL, NULL},
+                                {"collective", (PyCFunction)(void (*)(void))collective, METH_FASTCALL, NULL},
+                                {NULL, NULL, 0, NULL}};
+static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fastcall", NULL, -1, methods, NULL, NULL, NULL, NULL};
+
+PyMODINIT_FUNC PyInit__fastcall(void)
+{
+    s_data_ptr = PyUnicode_InternFromString("data_ptr");
+    s_ctypes = PyUnicode_InternFromString("ctypes");
+    s_data = PyUnicode_InternFromString("data");
+    return PyModule_Create(&module);
+}

@@ -12,7 +12,12 @@ from .. import _lib as L
 from ..utils.dtypes import data_ptr, hccl_dtype, numel
 
 
+_U64 = np.dtype(np.uint64)
+
+
 def _u64(a):
+    if type(a) is np.ndarray and a.dtype is _U64 and a.flags.c_contiguous:
+        return a
     return np.ascontiguousarray(np.asarray(a, dtype=np.uint64))
 
 
@@ -122,24 +127,20 @@ class Communicator:
 
     def collective(self, coll, send, recv, count, dtype, op=L.SUM, root=0, algo=L.ALGO_AUTO, nchan=0, counts=None,
                    displs=None, rows=None, stream=None):
-        o = L.B200Op()
-        o.coll, o.algo, o.nchan, o.dataType, o.op, o.root, o.count = coll, algo, nchan, dtype, op, root, int(count)
-        keep = []
+        tables = None
         if counts is not None:
-            c, d = _u64(counts), _u64(displs)
-            keep += [c, d]
-            o.counts, o.displs = c.ctypes.data, d.ctypes.data
+            tables = (_u64(counts), _u64(displs))
         if rows is not None:
-            sc, sd, rc, rd = [_u64(r) for r in rows]
-            keep += [sc, sd, rc, rd]
-            o.sendCounts, o.sdispls, o.recvCounts, o.rdispls = sc.ctypes.data, sd.ctypes.data, rc.ctypes.data, rd.ctypes.data
-        if coll == L.BARRIER:
-            sa = ra = None
+            tables = (_u64(rows[0]), _u64(rows[1]), _u64(rows[2]), _u64(rows[3]))
+        if not self.device:
+            st = None
+        elif stream is None:
+            st = _raw_stream()
         else:
-            sa, _ = self._bufs(send)
-            ra, _ = self._bufs(recv)
-        code = L.lib().HcclB200Collective(self._h, C.byref(o), sa, ra, self._stream(stream))
-        L.check(code, "HcclB200Collective(%d)" % coll)
+            st = stream if isinstance(stream, int) else stream.cuda_stream
+        code = L.fast.collective(self._h.value or 0, self.nlocal, coll, algo, nchan, dtype, op, root, int(count), send, recv, st, tables)
+        if code:
+            L.check(code, "HcclB200Collective(%d)" % coll)
 
     def repeat(self, coll, send, recv, count, dtype, iters, stride_bytes=0, nwin=1, op=L.SUM, root=0, algo=L.ALGO_AUTO, nchan=0,
                stream=None):
@@ -435,17 +436,21 @@ class Communicator:
         return self._h
 
 
-_RAW = None
+_RAW = _DEV = None
 
 
 def _raw_stream():
-    """Raw handle of torch's current CUDA stream (the cheap private accessor when it exists)."""
-    global _RAW
+    """Raw handle of torch's current CUDA stream (the cheap private accessors when they exist)."""
+    global _RAW, _DEV
+    if _RAW:
+        return _RAW(_DEV())
     import torch
     if _RAW is None:
+        torch.cuda.current_device()  # brings CUDA up if nothing has yet
         _RAW = getattr(torch._C, "_cuda_getCurrentRawStream", False)
-    if _RAW:
-        return _RAW(torch.cuda.current_device())
+        _DEV = torch._C._cuda_getDevice if _RAW else None
+        if _RAW:
+            return _RAW(_DEV())
     return torch.cuda.current_stream().cuda_stream
 
 
