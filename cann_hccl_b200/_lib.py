@@ -83,6 +83,12 @@ class B200Status(C.Structure):
                 ("tail", C.c_uint64)]
 
 
+class MoeLayer(C.Structure):
+    _fields_ = [("tokens", C.c_int64), ("capacityRows", C.c_int64), ("topk", C.c_int32), ("hidden", C.c_int32), ("nExperts", C.c_int32),
+                ("reserved", C.c_int32)] + [(n, C.c_void_p * 16) for n in ("rows", "pos", "dstRow", "expertOffsets", "recvRows", "overflow")] + \
+               [("scratch", C.c_void_p)]
+
+
 _lib = None
 fast = None  # csrc/python/fastcall.c, bound to the loaded library
 
@@ -161,6 +167,8 @@ def lib():
         "HcclB200MoeCount": [vp, C.c_int64, i32, vp, vp, vp],
         "HcclB200MoeOffsets": [vp, i32, i32, i32, vp, vp, vp, C.c_int64, vp, vp],
         "HcclB200MoeDispatch": [vp, vp, vp, vp, C.c_int64, i32, i32, i32, i32, i32, i32, P(vp), vp, C.c_int64, vp],
+        "HcclB200MoeDispatchLocal": [vp, P(MoeLayer), P(vp), P(vp), vp],
+        "HcclB200MoeCombineLocal": [vp, P(MoeLayer), P(vp), P(vp), P(vp), P(vp), vp],
         "HcclB200MoeCombine": [P(vp), vp, vp, vp, C.c_int64, i32, i32, i32, i32, i32, i32, vp, C.c_int64, vp],
         "HcclB200GemmBf16": [vp, vp, vp, i32, i32, i32, vp],
         "HcclB200GemmLaunchCounts": [P(u64), P(u64)],
@@ -211,6 +219,8 @@ def lib():
         fn = getattr(L, name)
         fn.argtypes = args
         fn.restype = C.c_int
+    L.HcclB200MoeScratchBytes.argtypes = [i32, C.c_int64, i32, i32]
+    L.HcclB200MoeScratchBytes.restype = C.c_int64
     L.HcclGetErrorString.argtypes = [C.c_int]
     L.HcclGetErrorString.restype = C.c_char_p
     L.HcclB200GetLastError.argtypes = []
@@ -222,7 +232,7 @@ def lib():
     loader = ExtensionFileLoader("_fastcall", _build.fastcall_path())
     fast = module_from_spec(spec_from_loader("_fastcall", loader))
     loader.exec_module(fast)
-    fast.bind(C.cast(L.HcclB200Collective, vp).value)
+    fast.bind(*[C.cast(f, vp).value for f in (L.HcclB200Collective, L.HcclB200MoeDispatchLocal, L.HcclB200MoeCombineLocal)])
     _lib = L
     return L
 

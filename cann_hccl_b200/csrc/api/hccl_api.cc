@@ -708,6 +708,38 @@ HcclResult HcclB200MoeCombine(void *const *yPeers, const int32_t *topkIdx, const
     CHK_RET_LOG(!yPeers || !topkIdx || !gates || !dstRow || !out, HCCL_E_PTR, "[EI0003] HcclB200MoeCombine: null pointer");
     return moe_combine(yPeers, topkIdx, gates, dstRow, tokens, topk, hidden, nExperts, nRanks, rank, pairwise, out, capacityRows, stream);
 }
+int64_t HcclB200MoeScratchBytes(int32_t nRanks, int64_t tokens, int32_t topk, int32_t nExperts)
+{
+    return nRanks < 1 || tokens < 0 || topk < 1 || nExperts < 1 ? -1 : moe_local_scratch_words(nRanks, tokens, topk, nExperts) * 4;
+}
+static HcclResult moe_layer(Communicator *c, const HcclB200MoeLayer *l, const char *api, MoeLocalLayer *out)
+{
+    CHK_RET_LOG(!l, HCCL_E_PTR, "[EI0003] %s: layer is null", api);
+    CHK_RET_LOG(c->transport() != TR_DEVICE || c->nlocal() != c->nranks() || l->nExperts > kMoeLocalMaxExperts, HCCL_E_NOT_SUPPORT,
+                "%s needs every rank of the communicator in this process on one GPU and at most %d experts", api, kMoeLocalMaxExperts);
+    *out = MoeLocalLayer{l->tokens, l->capacityRows, c->nranks(), l->topk, l->hidden, l->nExperts, l->pos, l->dstRow, l->expertOffsets, l->recvRows,
+                         l->overflow, l->scratch};
+    return HCCL_SUCCESS;
+}
+HcclResult HcclB200MoeDispatchLocal(HcclComm comm, const HcclB200MoeLayer *layer, void *const *x, void *const *topkIdx, aclrtStream stream)
+{
+    GET_COMM("HcclB200MoeDispatchLocal");
+    CHK_RET_LOG(!x || !topkIdx, HCCL_E_PTR, "[EI0003] HcclB200MoeDispatchLocal: null pointer");
+    MoeLocalLayer l;
+    CHK_RET(moe_layer(c, layer, "HcclB200MoeDispatchLocal", &l));
+    CHK_RET(c->ready());
+    return moe_local_dispatch(l, layer->rows, (const void *const *)x, (const int32_t *const *)topkIdx, stream);
+}
+HcclResult HcclB200MoeCombineLocal(HcclComm comm, const HcclB200MoeLayer *layer, void *const *rows, void *const *topkIdx, void *const *gates,
+                                   void *const *out, aclrtStream stream)
+{
+    GET_COMM("HcclB200MoeCombineLocal");
+    CHK_RET_LOG(!topkIdx || !gates || !out, HCCL_E_PTR, "[EI0003] HcclB200MoeCombineLocal: null pointer");
+    MoeLocalLayer l;
+    CHK_RET(moe_layer(c, layer, "HcclB200MoeCombineLocal", &l));
+    CHK_RET(c->ready());
+    return moe_local_combine(l, rows ? rows : layer->rows, (const int32_t *const *)topkIdx, (const float *const *)gates, out, stream);
+}
 HcclResult HcclB200GemmBf16(const void *A, const void *B, void *C, int32_t M, int32_t N, int32_t K, aclrtStream stream)
 {
     CHK_RET_LOG(!A || !B || !C, HCCL_E_PTR, "[EI0003] HcclB200GemmBf16: null pointer");

@@ -103,6 +103,7 @@ public:
     CostModel &cost_model() { return model_; }
 
     HcclResult collective(const OpRequest &rq);
+    HcclResult ready() { std::lock_guard<std::mutex> lk(op_mu_); return check_ready(); }  // takes operations: not suspended, no failure on record
     // Send/Recv between two ranks.  Exactly one side per call on ordinary communicators; on all-local communicators
     // both sides are given and run together.
     HcclResult send(const void *buf, uint64_t count, int dtype, int dest, void *stream);

@@ -3,7 +3,6 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstring>
-#include "common/log.h"
 #include "kernels/local_coll.cuh"
 
 namespace hcclb {
@@ -105,21 +104,6 @@ __global__ void __launch_bounds__(kLocalThreads) local_copy_kernel(const __grid_
     }
 }
 
-HcclResult launch_pdl(const void *fn, unsigned grid, void *args, void *stream, const char *what)
-{
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(kLocalThreads); cfg.stream = (cudaStream_t)stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at; cfg.numAttrs = 1;
-    void *kargs[] = {args};
-    cudaError_t e = cudaLaunchKernelExC(&cfg, fn, kargs);
-    if (e != cudaSuccess) { HLOG_ERROR("%s launch failed (%u CTAs): %s", what, grid, cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
-    return HCCL_SUCCESS;
-}
-
 // Vectors per tile: full unrolling where that still leaves a few CTAs for every SM, one vector per thread where it does not
 // (a small message is latency-bound: more CTAs with one load each finish sooner than fewer with many).
 uint32_t tile_vecs_for(uint64_t total_vecs, uint32_t full)
@@ -136,7 +120,7 @@ template <int JOBS> HcclResult launch_copy(LocalCopy &c, uint32_t tile_vecs, uns
     memcpy(a.job, c.job, sizeof(LocalCopyJob) * c.njobs);
     a.njobs = c.njobs;
     a.tile_vecs = tile_vecs;
-    return launch_pdl((const void *)local_copy_kernel<JOBS>, tiles, &a, stream, "direct copy");
+    return launch_pdl((const void *)local_copy_kernel<JOBS>, dim3(tiles), kLocalThreads, 0, &a, stream, "direct copy");
 }
 
 }  // namespace
@@ -184,7 +168,7 @@ HcclResult launch_local_reduce(LocalReduce &r, int dtype, int redop, void *strea
     r.njobs = n;
     if (tiles == 0) return HCCL_SUCCESS;
     if (tiles > 0x7fffffffu) return HCCL_E_PARA;
-    return launch_pdl(fn, (unsigned)tiles, &r, stream, "direct reduction");
+    return launch_pdl(fn, dim3((unsigned)tiles), kLocalThreads, 0, &r, stream, "direct reduction");
 }
 
 }  // namespace hcclb

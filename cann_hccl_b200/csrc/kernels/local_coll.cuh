@@ -2,15 +2,11 @@
 #pragma once
 #include "kernels/exec_plan_impl.cuh"
 #include "kernels/local_coll.h"
+#include "kernels/pdl.cuh"
 
 namespace hcclb {
 
 constexpr int kLocalThreads = 256;
-
-// Programmatic dependent launch: the next kernel of the stream may take the SM slots that this one leaves free, and waits
-// there; its launch latency and block scheduling hide behind this kernel's tail.  Nothing is read or written before pdl_wait().
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // 16 bytes at v0 + s (0 < s < 16), v0 and v1 being the two aligned vectors that hold them.  s is uniform in a job.
 __device__ __forceinline__ uint4 merge16(uint4 v0, uint4 v1, uint32_t s)

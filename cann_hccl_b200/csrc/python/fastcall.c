@@ -11,7 +11,11 @@
 #define MAX_LOCAL 16
 
 typedef HcclResult (*collective_fn)(HcclComm, const HcclB200Op *, void *const *, void *const *, aclrtStream);
+typedef HcclResult (*dispatch_fn)(HcclComm, const HcclB200MoeLayer *, void *const *, void *const *, aclrtStream);
+typedef HcclResult (*combine_fn)(HcclComm, const HcclB200MoeLayer *, void *const *, void *const *, void *const *, void *const *, aclrtStream);
 static collective_fn g_collective;
+static dispatch_fn g_dispatch;
+static combine_fn g_combine;
 static PyObject *s_data_ptr, *s_ctypes, *s_data;
 
 /* address of a tensor (data_ptr()) or numpy array (ctypes.data); None is null */
@@ -57,11 +61,13 @@ static int words(PyObject *x, Py_buffer *view, const uint64_t **out)
     return 0;
 }
 
-/* bind(address of HcclB200Collective) */
+/* bind(addresses of HcclB200Collective, HcclB200MoeDispatchLocal, HcclB200MoeCombineLocal) */
 static PyObject *bind(PyObject *self, PyObject *const *a, Py_ssize_t n)
 {
-    if (n != 1) { PyErr_SetString(PyExc_TypeError, "bind() takes one address"); return NULL; }
+    if (n != 3) { PyErr_SetString(PyExc_TypeError, "bind() takes 3 addresses"); return NULL; }
     g_collective = (collective_fn)PyLong_AsVoidPtr(a[0]);
+    g_dispatch = (dispatch_fn)PyLong_AsVoidPtr(a[1]);
+    g_combine = (combine_fn)PyLong_AsVoidPtr(a[2]);
     if (PyErr_Occurred()) return NULL;
     Py_RETURN_NONE;
 }
@@ -104,7 +110,43 @@ fail:
     return NULL;
 }
 
+/* moe_dispatch(comm, nlocal, layer, x, topk_idx, stream) -> result code */
+static PyObject *moe_dispatch(PyObject *self, PyObject *const *a, Py_ssize_t n)
+{
+    if (n != 6 || !g_dispatch) { PyErr_SetString(PyExc_TypeError, "moe_dispatch() takes 6 arguments, after bind()"); return NULL; }
+    void *comm = PyLong_AsVoidPtr(a[0]), *layer = PyLong_AsVoidPtr(a[2]), *stream = PyLong_AsVoidPtr(a[5]);
+    const Py_ssize_t nlocal = PyLong_AsSsize_t(a[1]);
+    if (PyErr_Occurred()) return NULL;
+    if (nlocal < 1 || nlocal > MAX_LOCAL) { PyErr_SetString(PyExc_ValueError, "bad number of local ranks"); return NULL; }
+    void *x[MAX_LOCAL], *idx[MAX_LOCAL];
+    if (addresses(a[3], nlocal, x) || addresses(a[4], nlocal, idx)) return NULL;
+    HcclResult rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = g_dispatch((HcclComm)comm, (const HcclB200MoeLayer *)layer, x, idx, (aclrtStream)stream);
+    Py_END_ALLOW_THREADS
+    return PyLong_FromLong((long)rc);
+}
+
+/* moe_combine(comm, nlocal, layer, rows (address of a table, 0: the layer's), topk_idx, gates, out, stream) -> result code */
+static PyObject *moe_combine(PyObject *self, PyObject *const *a, Py_ssize_t n)
+{
+    if (n != 8 || !g_combine) { PyErr_SetString(PyExc_TypeError, "moe_combine() takes 8 arguments, after bind()"); return NULL; }
+    void *comm = PyLong_AsVoidPtr(a[0]), *layer = PyLong_AsVoidPtr(a[2]), *rows = PyLong_AsVoidPtr(a[3]), *stream = PyLong_AsVoidPtr(a[7]);
+    const Py_ssize_t nlocal = PyLong_AsSsize_t(a[1]);
+    if (PyErr_Occurred()) return NULL;
+    if (nlocal < 1 || nlocal > MAX_LOCAL) { PyErr_SetString(PyExc_ValueError, "bad number of local ranks"); return NULL; }
+    void *idx[MAX_LOCAL], *gates[MAX_LOCAL], *out[MAX_LOCAL];
+    if (addresses(a[4], nlocal, idx) || addresses(a[5], nlocal, gates) || addresses(a[6], nlocal, out)) return NULL;
+    HcclResult rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = g_combine((HcclComm)comm, (const HcclB200MoeLayer *)layer, (void *const *)rows, idx, gates, out, (aclrtStream)stream);
+    Py_END_ALLOW_THREADS
+    return PyLong_FromLong((long)rc);
+}
+
 static PyMethodDef methods[] = {{"bind", (PyCFunction)(void (*)(void))bind, METH_FASTCALL, NULL},
+                                {"moe_dispatch", (PyCFunction)(void (*)(void))moe_dispatch, METH_FASTCALL, NULL},
+                                {"moe_combine", (PyCFunction)(void (*)(void))moe_combine, METH_FASTCALL, NULL},
                                 {"collective", (PyCFunction)(void (*)(void))collective, METH_FASTCALL, NULL},
                                 {NULL, NULL, 0, NULL}};
 static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fastcall", NULL, -1, methods, NULL, NULL, NULL, NULL};

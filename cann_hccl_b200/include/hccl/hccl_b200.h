@@ -77,6 +77,24 @@ extern HcclResult HcclB200MoeDispatch(const void *x, const int32_t *topkIdx, con
 extern HcclResult HcclB200MoeCombine(void *const *yPeers, const int32_t *topkIdx, const float *gates, const int32_t *dstRow, int64_t tokens,
                                      int32_t topk, int32_t hidden, int32_t nExperts, int32_t nRanks, int32_t rank, int32_t pairwise, void *out,
                                      int64_t capacityRows, aclrtStream stream);
+/* The same exchange for a communicator whose ranks are all in this process on one GPU (one rank included): counting, row bases
+ * and dispatch of every rank in two launches, combine of every rank in one, ordered by the stream.  The tables hold one device
+ * pointer per rank and stay the caller's; `scratch` has HcclB200MoeScratchBytes() bytes, zero before the first call, and
+ * belongs to one exchange (one stream at a time).  HCCL_E_NOT_SUPPORT on other communicators or above 8192 experts. */
+typedef struct HcclB200MoeLayerDef {
+    int64_t tokens, capacityRows;       /* tokens of one rank, rows of one receive buffer */
+    int32_t topk, hidden, nExperts, reserved;
+    void *rows[16];                     /* receive buffers by owner (combine may be given other rows) */
+    int32_t *pos[16], *dstRow[16];      /* tokens * topk words each */
+    int32_t *expertOffsets[16];         /* nExperts / ranks + 1 words each */
+    int32_t *recvRows[16], *overflow[16];
+    int32_t *scratch;
+} HcclB200MoeLayer;
+extern int64_t HcclB200MoeScratchBytes(int32_t nRanks, int64_t tokens, int32_t topk, int32_t nExperts);
+extern HcclResult HcclB200MoeDispatchLocal(HcclComm comm, const HcclB200MoeLayer *layer, void *const *x, void *const *topkIdx, aclrtStream stream);
+/* rows: NULL for the layer's receive buffers, else the expert outputs by owner (same layout). */
+extern HcclResult HcclB200MoeCombineLocal(HcclComm comm, const HcclB200MoeLayer *layer, void *const *rows, void *const *topkIdx, void *const *gates,
+                                          void *const *out, aclrtStream stream);
 /* ---- fused tensor-parallel kernels (tcgen05 GEMM + NVLink transfer in one sm_100a kernel); bf16, weights [N, K] ---- */
 /* C[M,N] = A[M,K] * B[N,K]^T (no communication). M % 128 == 0, N % 256 == 0, K % 64 == 0. */
 extern HcclResult HcclB200GemmBf16(const void *A, const void *B, void *C, int32_t M, int32_t N, int32_t K, aclrtStream stream);

@@ -49,14 +49,37 @@ class MoEExchange:
         self.base, self.expert_offsets, self.recv_rows, self.overflow = mk(n_experts), mk(self.El + 1), mk(1), mk(1)
         self.dst_row = mk(tokens * topk)
         self._topk = None
+        self._layer = self._local_layer(device)
         self.ranks = list(range(self.p)) if self.nl > 1 else [comm.rank]
+
+    def _local_layer(self, device):
+        """Tables of the launches that serve all ranks at once, where all of them are in this process on one GPU."""
+        if not (self.comm.device and self.nl == self.p and self.E <= 8192):
+            return None
+        self._scratch = torch.zeros(L.lib().HcclB200MoeScratchBytes(self.p, self.T, self.k, self.E) // 4, device=device, dtype=torch.int32)
+        y = L.MoeLayer(tokens=self.T, capacityRows=self.cap, topk=self.k, hidden=self.H, nExperts=self.E, scratch=self._scratch.data_ptr())
+        for name, ts in (("rows", self.recv), ("pos", self.pos), ("dstRow", self.dst_row), ("expertOffsets", self.expert_offsets),
+                         ("recvRows", self.recv_rows), ("overflow", self.overflow)):
+            for r, t in enumerate(ts):
+                getattr(y, name)[r] = t.data_ptr()
+        self._out_rows = (C.c_void_p * 16)(*[t.data_ptr() for t in self.expert_out])
+        self._layer_ptr, self._out_ptr = C.addressof(y), C.addressof(self._out_rows)
+        return y
 
     def _l(self, x):
         return list(x) if isinstance(x, (list, tuple)) else [x]
 
     def dispatch(self, x, topk_idx, variant="mesh"):
-        lib, st = L.lib(), C.c_void_p(_raw_stream())
         xs, idx = self._l(x), self._l(topk_idx)
+        if self._layer is not None:  # no links between the ranks: the variants, which order the traffic on them, are one
+            for t, i in zip(xs, idx):
+                assert i.dtype == torch.int32 and i.is_contiguous() and t.dtype == torch.bfloat16 and t.is_contiguous()
+            L.check(L.fast.moe_dispatch(self.comm.handle.value or 0, self.nl, self._layer_ptr, xs, idx, _raw_stream()), "HcclB200MoeDispatchLocal")
+            self._topk = idx
+            one = self.nl == 1
+            return (self.recv[0] if one else self.recv, self.expert_offsets[0] if one else self.expert_offsets,
+                    self.recv_rows[0] if one else self.recv_rows)
+        lib, st = L.lib(), C.c_void_p(_raw_stream())
         pw = 1 if variant == "pairwise" else 0
         for l in range(self.nl):
             assert idx[l].dtype == torch.int32 and idx[l].is_contiguous() and xs[l].dtype == torch.bfloat16 and xs[l].is_contiguous()
@@ -81,8 +104,16 @@ class MoEExchange:
 
     def combine(self, gates, variant="mesh", source="expert_out", out=None):
         """gates: fp32 [tokens, topk].  source: 'expert_out' (after the experts ran) or 'recv' (identity experts)."""
-        lib, st = L.lib(), C.c_void_p(_raw_stream())
         gs = self._l(gates)
+        if self._layer is not None:
+            outs = self._l(out) if out is not None else [torch.empty(self.T, self.H, device=g.device, dtype=torch.bfloat16) for g in gs]
+            for g in gs:
+                assert g.dtype == torch.float32 and g.is_contiguous()
+            rows = self._out_ptr if source == "expert_out" else 0
+            L.check(L.fast.moe_combine(self.comm.handle.value or 0, self.nl, self._layer_ptr, rows, self._topk, gs, outs, _raw_stream()),
+                    "HcclB200MoeCombineLocal")
+            return outs[0] if self.nl == 1 else outs
+        lib, st = L.lib(), C.c_void_p(_raw_stream())
         tab = self.out_tab if source == "expert_out" else self.recv_tab
         outs = self._l(out) if out is not None else [torch.empty(self.T, self.H, device=gs[0].device, dtype=torch.bfloat16) for _ in range(self.nl)]
         pw = 1 if variant == "pairwise" else 0

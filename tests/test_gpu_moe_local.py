@@ -1,0 +1,80 @@
+"""MoE exchange of all ranks in one process: the launches that serve every rank at once, and the per-rank launches that
+communicators over several processes take, against the plain PyTorch statement."""
+import pytest
+
+torch = pytest.importorskip("torch")
+import cann_hccl_b200 as H  # noqa: E402
+from cann_hccl_b200 import _lib as L  # noqa: E402
+from cann_hccl_b200.parallel import moe  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+# tokens x top-k around the chunk of 1024 pairs and beyond 32 chunks; top-k around the batch of eight rows; rows shorter than a
+# CTA, and longer than its four vectors per thread
+@pytest.mark.parametrize("p,T,hidden,E,k", [(1, 1, 8, 4, 1), (1, 127, 264, 16, 8), (2, 129, 256, 64, 8), (3, 257, 2048, 33, 9), (4, 100, 8456, 8, 2),
+                                            (1, 4100, 64, 256, 8), (8, 40, 512, 128, 17)])
+@pytest.mark.parametrize("per_rank", [False, True])
+def test_exchange(p, T, hidden, E, k, per_rank):
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    cfg = L.CommConfig.default()
+    cfg.hcclBufferSize = 2
+    c = H.Communicator.init_local(p, device=True, device_id=0, config=cfg)
+    ex = moe.MoEExchange(c, T, hidden, E, k, capacity_factor=float(p))
+    assert ex._layer is not None
+    if per_rank:
+        ex._layer = None
+    g = torch.Generator(device="cuda").manual_seed(T)
+    xs = [torch.randn(T, hidden, device="cuda", generator=g).to(torch.bfloat16) for _ in range(p)]
+    idx, gates = map(list, zip(*[moe.route(T, E, k, 7, r) for r in range(p)]))
+    idx[0][0, 0] = -1                                            # a slot without an expert is skipped
+    for _ in range(2):                                            # the second call finds the scratch as the first left it
+        ex.dispatch(xs if p > 1 else xs[0], idx if p > 1 else idx[0])
+        assert c.sync() == 0, c.describe_status()
+        El = E // p
+        for r in range(p):
+            want = torch.stack([sum((idx[s] == r * El + e).sum() for s in range(p)) for e in range(El)])
+            offs = ex.expert_offsets[r].long()
+            assert torch.equal(offs[1:] - offs[:-1], want) and int(offs[0]) == 0
+            assert int(ex.recv_rows[r]) == int(want.sum()) and int(ex.overflow[r]) == 0
+            for s in range(p):                                    # every pair's row is where dst_row says, and rows are not shared
+                mine = (idx[s] >= r * El) & (idx[s] < (r + 1) * El)
+                rows = ex.dst_row[s].view(T, k)[mine].long()
+                assert torch.equal(ex.recv[r][rows], xs[s].repeat_interleave(mine.sum(1), dim=0))
+            taken = torch.cat([ex.dst_row[s].view(T, k)[(idx[s] >= r * El) & (idx[s] < (r + 1) * El)] for s in range(p)])
+            assert taken.unique().numel() == taken.numel()
+            ex.expert_out[r].copy_(-ex.recv[r])
+        outs = ex.combine(gates if p > 1 else gates[0])
+        same = ex.combine(gates if p > 1 else gates[0], source="recv")
+        assert c.sync() == 0, c.describe_status()
+        outs, same = (outs, same) if p > 1 else ([outs], [same])
+        for r in range(p):
+            want = xs[r].float() * (gates[r] * (idx[r] >= 0)).sum(1, keepdim=True)
+            # k products summed in fp32 (batches of eight are rounded to bf16 in between on the per-rank path), one bf16 rounding
+            tol = 2.0 ** -8 * (1 + (k - 1) // 8)
+            assert bool(((same[r].float() - want).abs() <= tol * xs[r].float().abs() + 1e-6).all())
+            assert torch.equal(outs[r], -same[r])
+    ex.close()
+    c.destroy()
+
+
+def test_rows_beyond_the_capacity_are_dropped():
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    c = H.Communicator.init_root(1, H.Communicator.get_root_info(), 0, device=True)
+    T, hidden, E, k = 256, 64, 8, 2
+    ex = moe.MoEExchange(c, T, hidden, E, k, capacity_factor=0.5)
+    guard = ex.expert_out[0].fill_(3)
+    x = torch.randn(T, hidden, device="cuda").to(torch.bfloat16)
+    idx, gates = moe.route(T, E, k, 7, 0)
+    ex.dispatch(x, idx)
+    out = ex.combine(gates, source="recv")
+    assert c.sync() == 0
+    assert int(ex.overflow[0]) == 1 and int(ex.recv_rows[0]) == T * k
+    kept = (ex.dst_row[0].view(T, k) < ex.cap).float()
+    want = x.float() * (gates * kept).sum(1, keepdim=True)
+    assert bool(((out.float() - want).abs() <= 2.0 ** -8 * x.float().abs() + 1e-6).all())
+    assert bool((guard == 3).all())
+    ex.close()
+    c.destroy()
