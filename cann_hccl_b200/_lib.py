@@ -171,6 +171,8 @@ def lib():
         "HcclB200MoeCombineLocal": [vp, P(MoeLayer), P(vp), P(vp), P(vp), P(vp), vp],
         "HcclB200MoeCombine": [P(vp), vp, vp, vp, C.c_int64, i32, i32, i32, i32, i32, i32, vp, C.c_int64, vp],
         "HcclB200GemmBf16": [vp, vp, vp, i32, i32, i32, vp],
+        "HcclB200GemmBf16Act": [vp, vp, vp, i32, i32, i32, i32, vp],
+        "HcclB200AllGatherMatmulAct": [vp, P(vp), P(vp), P(vp), i32, i32, i32, i32, vp],
         "HcclB200GemmLaunchCounts": [P(u64), P(u64)],
         "HcclB200AllGatherMatmul": [vp, P(vp), P(vp), P(vp), i32, i32, i32, vp],
         "HcclB200MatmulReduceScatter": [vp, P(vp), P(vp), P(vp), i32, i32, i32, vp],

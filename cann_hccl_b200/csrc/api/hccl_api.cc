@@ -20,6 +20,7 @@
 #include "core/topo_probe.h"
 #include "health/consistency.h"
 #include "health/fault_inject.h"
+#include "kernels/fused/gemm_local.h"
 #include "kernels/moe_a2a.h"
 
 using namespace hcclb;
@@ -740,10 +741,20 @@ HcclResult HcclB200MoeCombineLocal(HcclComm comm, const HcclB200MoeLayer *layer,
     CHK_RET(c->ready());
     return moe_local_combine(l, rows ? rows : layer->rows, (const int32_t *const *)topkIdx, (const float *const *)gates, out, stream);
 }
-HcclResult HcclB200GemmBf16(const void *A, const void *B, void *C, int32_t M, int32_t N, int32_t K, aclrtStream stream)
+static HcclResult check_act(int32_t act, const char *api)
+{
+    CHK_RET_LOG(act < GEMM_ACT_NONE || act > GEMM_ACT_GELU, HCCL_E_PARA, "%s: unknown activation %d", api, act);
+    return HCCL_SUCCESS;
+}
+HcclResult HcclB200GemmBf16Act(const void *A, const void *B, void *C, int32_t M, int32_t N, int32_t K, int32_t act, aclrtStream stream)
 {
     CHK_RET_LOG(!A || !B || !C, HCCL_E_PTR, "[EI0003] HcclB200GemmBf16: null pointer");
-    return gemm_bf16_plain(A, B, C, M, N, K, stream);
+    CHK_RET(check_act(act, "HcclB200GemmBf16Act"));
+    return gemm_bf16_plain(A, B, C, M, N, K, act, stream);
+}
+HcclResult HcclB200GemmBf16(const void *A, const void *B, void *C, int32_t M, int32_t N, int32_t K, aclrtStream stream)
+{
+    return HcclB200GemmBf16Act(A, B, C, M, N, K, GEMM_ACT_NONE, stream);
 }
 HcclResult HcclB200GemmLaunchCounts(uint64_t *single, uint64_t *pair)
 {
@@ -751,12 +762,18 @@ HcclResult HcclB200GemmLaunchCounts(uint64_t *single, uint64_t *pair)
     tp_gemm_launch_counts(single, pair);
     return HCCL_SUCCESS;
 }
-HcclResult HcclB200AllGatherMatmul(HcclComm comm, void *const *xShards, void *const *weights, void *const *outs, int32_t M, int32_t N, int32_t K,
-                                   aclrtStream stream)
+HcclResult HcclB200AllGatherMatmulAct(HcclComm comm, void *const *xShards, void *const *weights, void *const *outs, int32_t M, int32_t N, int32_t K,
+                                      int32_t act, aclrtStream stream)
 {
     GET_COMM("HcclB200AllGatherMatmul");
     CHK_RET_LOG(!xShards || !weights || !outs, HCCL_E_PTR, "[EI0003] HcclB200AllGatherMatmul: null pointer");
-    return c->tp_all_gather_matmul((const void *const *)xShards, (const void *const *)weights, outs, M, N, K, stream);
+    CHK_RET(check_act(act, "HcclB200AllGatherMatmulAct"));
+    return c->tp_all_gather_matmul((const void *const *)xShards, (const void *const *)weights, outs, M, N, K, act, stream);
+}
+HcclResult HcclB200AllGatherMatmul(HcclComm comm, void *const *xShards, void *const *weights, void *const *outs, int32_t M, int32_t N, int32_t K,
+                                   aclrtStream stream)
+{
+    return HcclB200AllGatherMatmulAct(comm, xShards, weights, outs, M, N, K, GEMM_ACT_NONE, stream);
 }
 HcclResult HcclB200MatmulReduceScatter(HcclComm comm, void *const *inputs, void *const *weights, void *const *outs, int32_t M, int32_t N,
                                        int32_t K, aclrtStream stream)

@@ -158,6 +158,7 @@ EnvConfig parse_env(const std::map<std::string, std::string> &v)
         else fail(c, "HCCL_PIPE_GROUPS must be a,b[,c] with values in [1,16]");
     }
     if (auto s = get("HCCL_PLAN_RACE_CHECK")) c.plan_race_check = *s == "1" || lower(*s) == "true";
+    if (auto s = get("HCCL_TP_DIRECT")) c.tp_direct = !(*s == "0" || lower(*s) == "false");
     if (auto s = get("HCCL_TP_GEMM_PAIR")) c.tp_gemm_pair = !(*s == "0" || lower(*s) == "false");
     if (auto s = get("HCCL_NCCL_LIB")) c.ncc_lib = *s;
     if (auto s = get("HCCL_WHITELIST_DISABLE")) c.whitelist_enable = *s == "0";

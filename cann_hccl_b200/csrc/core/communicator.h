@@ -145,9 +145,9 @@ public:
     uint64_t overflow_count();
 
     // Fused tensor-parallel operators (kernels/fused/tp_gemm_sm100.cu).  Pointers per local rank; bf16; weights [N, K].
-    //   all_gather_matmul:     y[M,N]     = all_gather(x_shard[M/p,K]) * w[N,K]^T
+    //   all_gather_matmul:     y[M,N]     = act(all_gather(x_shard[M/p,K]) * w[N,K]^T)        act: GemmAct, on the fp32 sums
     //   matmul_reduce_scatter: out[M/p,N] = reduce_scatter_rows(h[M,K] * w[N,K]^T)
-    HcclResult tp_all_gather_matmul(const void *const *x_shard, const void *const *w, void *const *y, int M, int N, int K, void *stream);
+    HcclResult tp_all_gather_matmul(const void *const *x_shard, const void *const *w, void *const *y, int M, int N, int K, int act, void *stream);
     HcclResult tp_matmul_reduce_scatter(const void *const *h, const void *const *w, void *const *out, int M, int N, int K, void *stream);
     // Selection only (no execution).
     Selection select(int coll, uint64_t count, int dtype, int redop) const;
@@ -189,6 +189,7 @@ private:
     bool zc_candidate(const OpRequest &rq) const;
     bool registered_send(const OpRequest &rq, int *handle, size_t *offset);
     int pipe_mode_for(int coll) const;  // PipeMode of a collective, -1 when it has no pipelined kernel
+    HcclResult tp_direct(int form, const void *const *a, const void *const *b, void *const *c, int M, int N, int K, int act, void *stream);
     HcclResult tp_workspace(const std::string &key, size_t data_bytes, int M, void **ws_out);
     void tp_release_workspaces();
     int overlap_kind(const OpRequest &rq, int li) const;
@@ -302,7 +303,7 @@ private:
 };
 
 // Plain tcgen05 GEMM C[M,N] = A[M,K] * B[N,K]^T in bf16 (no communicator needed).
-HcclResult gemm_bf16_plain(const void *A, const void *B, void *C, int M, int N, int K, void *stream);
+HcclResult gemm_bf16_plain(const void *A, const void *B, void *C, int M, int N, int K, int act, void *stream);
 // Launches of the fused GEMM kernels in this process: one CTA per tile / clusters of two CTAs per 256 x 256 tile.
 void tp_gemm_launch_counts(uint64_t *single, uint64_t *pair);
 // Device executor entry (kernels/exec_plan.cu).

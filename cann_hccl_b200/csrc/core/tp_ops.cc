@@ -5,8 +5,10 @@
 #include <cstdlib>
 #include <cstring>
 #include <sstream>
+#include "common/env.h"
 #include "common/log.h"
 #include "core/communicator.h"
+#include "kernels/fused/gemm_local.h"
 #include "kernels/fused/tp_gemm.h"
 
 namespace hcclb {
@@ -73,17 +75,28 @@ static void fill_common(TpGemmParams &P, int mode, int M, int N, int K, int rank
     P.status = status; P.fail_word = fail_word;
 }
 
-HcclResult gemm_bf16_plain(const void *A, const void *B, void *C, int M, int N, int K, void *stream)
+HcclResult gemm_bf16_plain(const void *A, const void *B, void *C, int M, int N, int K, int act, void *stream)
 {
-    TpGemmParams P;
-    fill_common(P, TP_MODE_PLAIN, M, N, K, 0, 1, 1, 10000000000ull, nullptr, nullptr);
-    P.C = (__nv_bfloat16 *)C;
-    P.ldc = N;
-    const void *a[1] = {A}, *b[1] = {B};
-    return launch_tp_gemm(&P, a, b, 1, 0, stream);
+    GemmCall g;
+    g.M = M; g.N = N; g.K = K; g.act = act;
+    g.A[0] = A; g.B[0] = B; g.C[0] = C;
+    return launch_gemm_local(g, nullptr, stream);
 }
 
-HcclResult Communicator::tp_all_gather_matmul(const void *const *x_shard, const void *const *w, void *const *y, int M, int N, int K, void *stream)
+// Every rank in this process on one GPU: nothing to transfer, one GEMM over all ranks' operands (kernels/fused/gemm_local.cu).
+HcclResult Communicator::tp_direct(int form, const void *const *a, const void *const *b, void *const *c, int M, int N, int K, int act, void *stream)
+{
+    GemmCall g;
+    g.form = nranks_ == 1 ? GEMM_PLAIN : form;
+    g.p = nranks_; g.M = M; g.N = N; g.K = K; g.act = act;
+    for (int r = 0; r < nranks_; ++r) { g.A[r] = a[r]; g.B[r] = b[r]; g.C[r] = c[r]; }
+    StateGuard guard(state_, CS_INUSE);
+    stats_.launches++;
+    stats_.ops[form == GEMM_GATHER ? COLL_ALLGATHER : COLL_REDUCE_SCATTER]++;
+    return launch_gemm_local(g, status_[0], stream);
+}
+
+HcclResult Communicator::tp_all_gather_matmul(const void *const *x_shard, const void *const *w, void *const *y, int M, int N, int K, int act, void *stream)
 {
     std::lock_guard<std::mutex> lk(op_mu_);
     CHK_RET(check_ready());
@@ -91,6 +104,7 @@ HcclResult Communicator::tp_all_gather_matmul(const void *const *x_shard, const 
     int nl = nlocal();
     CHK_RET_LOG(nl > kTpMaxLocal, HCCL_E_NOT_SUPPORT, "at most %d virtual ranks per GPU for the fused kernels", kTpMaxLocal);
     CHK_RET_LOG(M % (128 * nranks_) != 0, HCCL_E_PARA, "M (%d) must be a multiple of 128 x ranks (%d)", M, 128 * nranks_);
+    if (nl == nranks_ && env_config().tp_direct) return tp_direct(GEMM_GATHER, x_shard, w, y, M, N, K, act, stream);
     std::ostringstream key;
     key << "ag:" << M << ':' << K;
     void *wsp = nullptr;
@@ -118,6 +132,7 @@ HcclResult Communicator::tp_all_gather_matmul(const void *const *x_shard, const 
         fill_common(P[li], TP_MODE_AG, M, N, K, ctx_[li].rank, nranks_, ws.epoch, ctx_[li].timeout_ns, status_[li], ctx_[li].exit_counter + 1);
         P[li].C = (__nv_bfloat16 *)y[li];
         P[li].ldc = N;
+        P[li].act = act;
         P[li].x_shard = (const __nv_bfloat16 *)x_shard[li];
         for (int q = 0; q < nranks_; ++q) {
             P[li].flags[q] = (uint64_t *)ws.segs[li].peer[q];
@@ -146,12 +161,7 @@ HcclResult Communicator::tp_matmul_reduce_scatter(const void *const *h, const vo
     int nl = nlocal();
     CHK_RET_LOG(nl > kTpMaxLocal, HCCL_E_NOT_SUPPORT, "at most %d virtual ranks per GPU for the fused kernels", kTpMaxLocal);
     CHK_RET_LOG(M % (128 * nranks_) != 0, HCCL_E_PARA, "M (%d) must be a multiple of 128 x ranks (%d)", M, 128 * nranks_);
-    if (nranks_ == 1) {
-        // nothing to reduce or scatter: the product goes straight to the output, without a pass through a receive slot
-        stats_.launches++;
-        stats_.ops[COLL_REDUCE_SCATTER]++;
-        return gemm_bf16_plain(h[0], w[0], out[0], M, N, K, stream);
-    }
+    if (nl == nranks_ && (nranks_ == 1 || env_config().tp_direct)) return tp_direct(GEMM_REDUCE, h, w, out, M, N, K, GEMM_ACT_NONE, stream);
     std::ostringstream key;
     key << "rs:" << M << ':' << N << ':' << K;  // the panel layout of the completion counters depends on K as well
     void *wsp = nullptr;

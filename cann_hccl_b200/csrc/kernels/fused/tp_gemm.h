@@ -4,13 +4,13 @@
 #include <cuda_bf16.h>
 #include "algo/plan.h"
 namespace hcclb {
-enum TpMode : int { TP_MODE_PLAIN = 0, TP_MODE_AG = 1, TP_MODE_RS = 2 };
+enum TpMode : int { TP_MODE_AG = 1, TP_MODE_RS = 2 };
 constexpr int kTpMaxLocal = 4;   // virtual ranks of one GPU that one cooperative launch can run (single-GPU validation)
 struct alignas(64) TpGemmParams {
     CUtensorMap tmA, tmB;             // A [M,K] and B [N,K], both K-major bf16, this GPU's own memory
     CUtensorMap tmX;                  // AG: this rank's own shard [M/p, K] in the caller's buffer
-    __nv_bfloat16 *C;                 // PLAIN / AG: output [M, ldc]
-    int ldc;
+    __nv_bfloat16 *C;                 // AG: output [M, ldc]
+    int ldc, act;                     // act: GemmAct of the AG epilogue
     int M, N, K;
     int mode, rank, nranks;
     int n_gemm_ctas;                  // CTAs [0, n_gemm_ctas) compute; the rest move data
@@ -34,5 +34,6 @@ inline size_t tp_flag_words(int M, int nranks) { return (size_t)4 * nranks + (si
 // Fills the tensor maps and launches.  `A` / `B` per local rank.  n_comm_ctas data-movement CTAs per rank.
 HcclResult launch_tp_gemm(TpGemmParams *P, const void *const *A, const void *const *B, int nlocal, int n_comm_ctas, void *stream);
 size_t tp_gemm_smem_bytes();
+HcclResult tp_gemm_load();  // loads the kernels and their static scratch on the current device
 void tp_gemm_launch_counts(uint64_t *single, uint64_t *pair);
 }  // namespace hcclb

@@ -1,6 +1,5 @@
 // Fused tensor-parallel GEMM kernels for sm_100a (bf16 in, fp32 accumulate in TMEM, bf16 out).
 //
-//   mode PLAIN : C[M,N] = A[M,K] * B[N,K]^T                                   (building block, TP = 1)
 //   mode AG    : all-gather(X shards) -> Y = X * W^T   (column-parallel layer; X sharded by rows over the ranks)
 //   mode RS    : P = H * W^T -> reduce-scatter(P) by rows  (row-parallel layer; every rank ends with its row block)
 //
@@ -40,6 +39,7 @@
 #include "common/env.h"
 #include "common/log.h"
 #include "core/device_api.h"
+#include "kernels/fused/tc05.cuh"
 #include "kernels/fused/tp_gemm.h"
 #include "kernels/fused/tp_gemm_noalloc.h"
 #include "kernels/prims.cuh"
@@ -48,7 +48,7 @@ namespace hcclb {
 
 namespace {
 
-constexpr int BM = 128, BN = 256, BK = 64, UMMA_K = 16;
+using namespace tc05;
 constexpr int kStages = 4;
 constexpr int kStagesPair = 6;                        // pair variant: a stage holds 128 rows of A and 128 rows of B
 constexpr int kMaxStages = kStagesPair;
@@ -61,8 +61,6 @@ static_assert(kStagesPair * kStageBytesPair <= kStages * kStageBytes, "both vari
 constexpr uint32_t kTmemCols = 512;
 constexpr int kCommBuf = 32 * 1024, kCommDepth = 6;  // bulk-copy ring of a data-movement CTA (lives in the tile buffers)
 constexpr int kEpiCols = 64, kEpiStride = kEpiCols * 2 + 16;  // epilogue chunk: 64 bf16 per row, padded against bank conflicts
-constexpr uint64_t kPairWaitNs = 4000000000ull;     // pair variant: longest wait on a barrier that the other CTA completes
-constexpr uint32_t kSpinLimit = 1u << 28;            // iterations of an mbarrier poll before it gives up (seconds)
 
 struct SharedStorage {
     alignas(1024) uint8_t tiles[kStages * kStageBytes];
@@ -78,210 +76,6 @@ struct SharedStorage {
     uint32_t early_go[2];    // RS: decision of the early reducer's leader for its next item (by item parity)
     uint32_t early_count;    // RS: items this CTA's early reducer finished before the GEMM ended
 };
-
-// ---------------------------------------------------------------------------------------------- PTX wrappers
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    return ok != 0;
-}
-// Bounded wait: false when the limit ran out or another role already failed.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile uint32_t *fail)
-{
-    for (uint32_t it = 0; it < kSpinLimit; ++it) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((it & 1023) == 1023 && *fail) return false;
-    }
-    *fail = HCCL_E_TIMEOUT;
-    return false;
-}
-// Cluster-scope forms for the pair variant: barriers that the other CTA of the pair (its threads, its TMA loads or the
-// leader's multicast commits) completes.
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t *bar, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    return ok != 0;
-}
-template <bool kCluster>
-__device__ __forceinline__ bool mbar_wait_t(uint64_t *bar, uint32_t parity, volatile uint32_t *fail)
-{
-    if constexpr (!kCluster) {
-        return mbar_wait(bar, parity, fail);
-    } else {
-        // the other CTA of the pair learns of a failure only through its own waits: bound them by time, a few seconds
-        uint64_t t0 = 0;
-        for (uint32_t it = 0; it < kSpinLimit; ++it) {
-            if (mbar_try_wait_cluster(bar, parity)) return true;
-            if ((it & 1023) == 1023) {
-                if (*fail) return false;
-                const uint64_t now = global_timer_ns();
-                if (t0 == 0) t0 = now;
-                else if (now - t0 > kPairWaitNs) break;
-            }
-        }
-        *fail = HCCL_E_TIMEOUT;
-        return false;
-    }
-}
-__device__ __forceinline__ uint32_t cluster_ctarank()
-{
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-// Address of the same shared-memory location in CTA `rank` of this cluster (shared::cluster window).
-__device__ __forceinline__ uint32_t mapa_u32(uint32_t cta_addr, uint32_t rank)
-{
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(cta_addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr)
-{
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ void cluster_sync_all()
-{
-    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// TMA load of the pair variant: the data lands in this CTA's shared memory, the bytes are counted on the barrier at
-// `bar_cluster_addr`, which may belong to the other CTA of the pair (no multicast: one load, one destination).
-__device__ __forceinline__ void tma_load_2d_pair(void *dst, const CUtensorMap *map, uint32_t bar_cluster_addr, int x, int y)
-{
-    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-                 ::"r"(smem_u32(dst)), "l"(map), "r"(bar_cluster_addr), "r"(x), "r"(y) : "memory");
-}
-__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, uint64_t *bar, int x, int y)
-{
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-                 ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y) : "memory");
-}
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
-{
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void bulk_s2g(void *dst, const void *src, uint32_t bytes)
-{
-    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
-template <int N> __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory"); }
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
-__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ bool elect_one()
-{
-    uint32_t pred;
-    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(pred));
-    return pred != 0;
-}
-
-// Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, rows 128 bytes apart, 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t make_smem_desc(const void *ptr)
-{
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_u32(ptr) & 0x3FFFF) >> 4);   // start address, 16-byte units
-    d |= (uint64_t)1 << 16;                            // leading-dimension byte offset (unused for swizzled K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;                  // stride-dimension byte offset: 8 rows x 128 bytes
-    d |= (uint64_t)1 << 46;                            // descriptor version of sm_100
-    d |= (uint64_t)2 << 61;                            // SWIZZLE_128B
-    return d;
-}
-// Instruction descriptor: D fp32, A and B bf16, both K-major, N = 256, M = 128.
-constexpr uint32_t kInstrDesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-
-__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate)
-{
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n}"
-                 ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(kInstrDesc), "r"(accumulate), "r"(0u) : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint64_t *bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-// Pair variant: D fp32, A and B bf16 K-major, N = 256, M = 256 (128 rows per CTA); issued by one thread of the leader CTA.
-constexpr uint32_t kInstrDescPair = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
-__device__ __forceinline__ void umma_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate)
-{
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n}"
-                 ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(kInstrDescPair), "r"(accumulate), "r"(0u) : "memory");
-}
-// Arrives on the barrier at this offset in BOTH CTAs of the pair once the MMAs issued so far are complete.
-__device__ __forceinline__ void umma_commit_pair(uint64_t *bar)
-{
-    const uint16_t both = 3;
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(smem_u32(bar)), "h"(both) : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32])
-{
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,"
-        "%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
-          "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-          "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-__device__ __forceinline__ uint32_t pack_bf16(uint32_t a, uint32_t b)
-{
-    __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(a), __uint_as_float(b));
-    return *(uint32_t *)&v;
-}
-__device__ __forceinline__ void red_add_release_sys(uint64_t *p, uint64_t v)
-{
-    asm volatile("red.release.sys.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ void red_add_release_gpu(uint64_t *p, uint64_t v)
-{
-    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ void st_release_gpu(uint64_t *p, uint64_t v)
-{
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ uint64_t ld_acquire_gpu(const uint64_t *p)
-{
-    uint64_t v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-
-// Bounded wait on a global word (device or system scope); returns false after the time limit or a CTA failure.
-__device__ __forceinline__ bool wait_word_ge(const uint64_t *p, uint64_t want, bool sys, uint64_t deadline, volatile uint32_t *fail)
-{
-    for (uint32_t it = 0;; ++it) {
-        uint64_t v = sys ? ld_acquire_sys(p) : ld_acquire_gpu(p);
-        if (v >= want) return true;
-        if ((it & 63) == 63) {
-            if (*fail) return false;
-            if (global_timer_ns() > deadline) { *fail = HCCL_E_TIMEOUT; return false; }
-        }
-    }
-}
 
 __device__ __forceinline__ void report(const TpGemmParams &P, uint32_t code, int where)
 {
@@ -335,7 +129,7 @@ __device__ __forceinline__ void tile_coords(const TpGemmParams &P, int t, int n_
     const int r2 = r1 - panel * per_panel;
     const int ml = r2 / w;
     nt = n0 + r2 % w;
-    if (P.mode == TP_MODE_PLAIN || P.nranks == 1) { mt = ml; return; }
+    if (P.nranks == 1) { mt = ml; return; }
     if (P.mode == TP_MODE_RS) {  // the next rank's rows first so that remote partial tiles leave early; my own rows last
         mt = (ml + ((P.rank + 1) % P.nranks) * (m_tiles / P.nranks)) % m_tiles;
         return;
@@ -570,6 +364,15 @@ __device__ void reduce_tail_rs(const TpGemmParams &P, SharedStorage &S, int pw, 
     }
 }
 
+template <int ACT> __device__ __forceinline__ void activate64(uint32_t (&a)[32], uint32_t (&b)[32])
+{
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+        a[i] = __float_as_uint(activate<ACT>(__uint_as_float(a[i])));
+        b[i] = __float_as_uint(activate<ACT>(__uint_as_float(b[i])));
+    }
+}
+
 // ---------------------------------------------------------------------------------------------- the kernel
 // kPair: the CTAs 2i and 2i+1 form a cluster and share 256 x 256 tiles (see the head of the file).  A pair walks the tile
 // order in units of two m tiles: the tile coordinates are computed on a grid of m_tiles / 2 row blocks and CTA r of the pair
@@ -699,7 +502,7 @@ __device__ __forceinline__ void tp_gemm_body(const TpGemmParams &P, SharedStorag
         // ------------------------------------------------------------------ epilogue: TMEM -> registers -> bf16 -> global
         const int q4 = warp & 3;  // a warp may only touch the TMEM lane quarter given by its index modulo 4
         uint32_t tile_i = 0, owner_ok = 0;
-        const int per = P.nranks > 0 ? m_tiles / P.nranks : m_tiles;
+        const int per = m_tiles / P.nranks;
         for (int t = unit_first; t < units && !*fail; t += unit_step, ++tile_i) {
             int mt, nt, panel;
             unit_coords(t, mt, nt, panel);
@@ -730,6 +533,8 @@ __device__ __forceinline__ void tp_gemm_body(const TpGemmParams &P, SharedStorag
                 tmem_ld32(tmem_base + buf * BN + c0 + ((uint32_t)(q4 * 32) << 16), r0);
                 tmem_ld32(tmem_base + buf * BN + c0 + 32 + ((uint32_t)(q4 * 32) << 16), r1);
                 tmem_ld_wait();
+                if (P.act == GEMM_ACT_SILU) activate64<GEMM_ACT_SILU>(r0, r1);
+                else if (P.act == GEMM_ACT_GELU) activate64<GEMM_ACT_GELU>(r0, r1);
                 bulk_wait_read<0>();  // the previous piece has left the slot
                 uint4 *o = (uint4 *)slot;
 #pragma unroll
@@ -827,11 +632,19 @@ HcclResult encode_2d(CUtensorMap *map, const void *base, uint64_t rows, uint64_t
 
 size_t tp_gemm_smem_bytes() { return sizeof(SharedStorage) + 1024; }
 
+HcclResult tp_gemm_load()
+{
+    for (const void *fn : {(const void *)tp_gemm_pair_kernel, (const void *)tp_gemm_kernel})
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tp_gemm_smem_bytes()) != cudaSuccess) return HCCL_E_RUNTIME;
+    return HCCL_SUCCESS;
+}
+
 static std::atomic<uint64_t> g_launches[2];
 void tp_gemm_launch_counts(uint64_t *single, uint64_t *pair)
 {
-    *single = g_launches[0].load();
-    *pair = g_launches[1].load();
+    gemm_local_launch_counts(single, pair);
+    *single += g_launches[0].load();
+    *pair += g_launches[1].load();
 }
 
 HcclResult launch_tp_gemm(TpGemmParams *P, const void *const *A, const void *const *B, int nlocal, int n_comm_ctas, void *stream)
@@ -842,7 +655,7 @@ HcclResult launch_tp_gemm(TpGemmParams *P, const void *const *A, const void *con
         HLOG_ERROR("fused GEMM needs M %% %d == 0, N %% %d == 0, K %% %d == 0 (got %d x %d x %d)", BM, BN, BK, P0.M, P0.N, P0.K);
         return HCCL_E_PARA;
     }
-    if (P0.mode != TP_MODE_PLAIN && P0.nranks > 1 && (P0.M / BM) % P0.nranks) {
+    if (P0.nranks > 1 && (P0.M / BM) % P0.nranks) {
         HLOG_ERROR("fused GEMM needs the %d row blocks to divide evenly over %d ranks", P0.M / BM, P0.nranks);
         return HCCL_E_PARA;
     }
@@ -855,11 +668,10 @@ HcclResult launch_tp_gemm(TpGemmParams *P, const void *const *A, const void *con
     int per_rank = sms / nlocal;  // all CTAs of all local ranks must be resident together
     if (n_comm_ctas > per_rank / 4) n_comm_ctas = n_comm_ctas ? std::max(1, per_rank / 4) : 0;
     if (n_comm_ctas > kMaxCommCtas) n_comm_ctas = kMaxCommCtas;
-    // with communication every rank must run the same grid (completion counters count CTAs)
-    int total = (P0.M / BM) * (P0.N / BN);
+    // every rank must run the same grid (completion counters count CTAs)
     // pair variant (clusters of two CTAs on 256 x 256 tiles): every rank's rows must come in pairs of 128-row blocks.  The
     // choice depends on the shape and the environment only, so every rank makes the same one.
-    const int rows_per_rank = P0.mode == TP_MODE_PLAIN || P0.nranks < 1 ? P0.M : P0.M / P0.nranks;
+    const int rows_per_rank = P0.M / std::max(1, P0.nranks);
     const bool pair = env_config().tp_gemm_pair && rows_per_rank % (2 * BM) == 0 && per_rank >= 4;
     if (pair) {
         // clusters that can be resident together (a cluster needs both of its SMs inside one GPC): asked once per device
@@ -887,7 +699,7 @@ HcclResult launch_tp_gemm(TpGemmParams *P, const void *const *A, const void *con
         per_rank &= ~1;
         if (n_comm_ctas) n_comm_ctas = std::min((n_comm_ctas + 1) & ~1, std::max(2, (per_rank / 4) & ~1));
     }
-    int n_gemm = P0.mode == TP_MODE_PLAIN ? std::min(total, per_rank) : per_rank - n_comm_ctas;
+    const int n_gemm = per_rank - n_comm_ctas;
     TpGemmParamsArray arr;
     memset(&arr, 0, sizeof(arr));
     for (int i = 0; i < nlocal; ++i) {
@@ -918,9 +730,7 @@ HcclResult launch_tp_gemm(TpGemmParams *P, const void *const *A, const void *con
     dim3 grid((unsigned)(n_gemm + n_comm_ctas), (unsigned)nlocal), block(kThreads);
     // AG and RS mode make CTAs of one rank wait on each other (GEMM CTAs on the data-movement CTAs, the reduce tail on the
     // other CTAs' tiles): a cooperative launch guarantees that all of them are resident together even when another kernel
-    // shares the GPU.  The plain GEMM has no such dependency.
-    // (a single rank in AG mode has no data-movement CTAs and waits for nobody)
-    const bool coop = nlocal > 1 || P0.mode == TP_MODE_RS || (P0.mode == TP_MODE_AG && P0.nranks > 1);
+    // shares the GPU.
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = (cudaStream_t)stream;
@@ -931,15 +741,13 @@ HcclResult launch_tp_gemm(TpGemmParams *P, const void *const *A, const void *con
         attrs[na].val.clusterDim.x = 2; attrs[na].val.clusterDim.y = 1; attrs[na].val.clusterDim.z = 1;
         ++na;
     }
-    if (coop) {
-        attrs[na].id = cudaLaunchAttributeCooperative;
-        attrs[na].val.cooperative = 1;
-        ++na;
-    }
+    attrs[na].id = cudaLaunchAttributeCooperative;
+    attrs[na].val.cooperative = 1;
+    ++na;
     cfg.attrs = attrs; cfg.numAttrs = na;
     void *kargs[] = {(void *)&arr};
     cudaError_t e = cudaLaunchKernelExC(&cfg, fn, kargs);
-    if (e != cudaSuccess) { HLOG_ERROR("fused GEMM launch failed (%s%s): %s", pair ? "pair " : "", coop ? "cooperative" : "plain", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
+    if (e != cudaSuccess) { HLOG_ERROR("fused GEMM launch failed (%s): %s", pair ? "pairs" : "single CTAs", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
     g_launches[pair ? 1 : 0]++;
     return HCCL_SUCCESS;
 }

@@ -107,6 +107,11 @@ extern HcclResult HcclB200AllGatherMatmul(HcclComm comm, void *const *xShards, v
 /* Row-parallel layer: outs [M/p, N] = reduce_scatter_rows(inputs [M, K] * weights[N, K]^T). */
 extern HcclResult HcclB200MatmulReduceScatter(HcclComm comm, void *const *inputs, void *const *weights, void *const *outs, int32_t M,
                                               int32_t N, int32_t K, aclrtStream stream);
+/* The plain product and the column-parallel layer with an activation on the fp32 sums, before they are rounded to bf16:
+ * 0 none, 1 SiLU, 2 GELU (erf form). */
+extern HcclResult HcclB200GemmBf16Act(const void *A, const void *B, void *C, int32_t M, int32_t N, int32_t K, int32_t act, aclrtStream stream);
+extern HcclResult HcclB200AllGatherMatmulAct(HcclComm comm, void *const *xShards, void *const *weights, void *const *outs, int32_t M, int32_t N,
+                                             int32_t K, int32_t act, aclrtStream stream);
 /* In-kernel timestamps of the newest executor launch (needs HCCL_KERNEL_TRACE=1 at communicator creation):
  * out[0] = kernel start (globaltimer ns), then per step {after wait, after data movement, after signal}. */
 extern HcclResult HcclB200GetKernelTrace(HcclComm comm, uint32_t localRank, uint64_t *out, size_t capWords, int32_t *nsteps);

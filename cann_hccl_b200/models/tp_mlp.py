@@ -1,7 +1,7 @@
 """Tensor-parallel MLP block (Llama-style shapes) built on the fused kernels.
 
 The activations enter and leave sharded by rows (sequence-parallel layout): each rank holds [tokens/p, hidden].
-    h = act( all_gather(x) @ W_up[ffn/p, hidden].T )      one fused all-gather + GEMM kernel
+    h = act( all_gather(x) @ W_up[ffn/p, hidden].T )      one fused all-gather + GEMM kernel, act in its epilogue
     y = reduce_scatter( h @ W_down[hidden, ffn/p].T )     one fused GEMM + reduce-scatter kernel
 Weights are random (N(0, 0.02)); `reference_forward` is the plain PyTorch fp32 statement of the same math.
 """
@@ -15,7 +15,9 @@ class TensorParallelMLP:
         self.comm, self.hidden, self.ffn = comm, hidden, ffn
         p = comm.nranks
         assert ffn % p == 0
+        self.activation = activation
         self.act = {"silu": torch.nn.functional.silu, "gelu": torch.nn.functional.gelu, "none": lambda t: t}[activation]
+        self._epilogue_act = self.act
         g = torch.Generator(device=device).manual_seed(seed)
         # full weights are generated identically on every rank, then sliced: rank r owns rows / columns [r*ffn/p, (r+1)*ffn/p)
         w_up = (torch.randn(ffn, hidden, device=device, generator=g) * 0.02).to(torch.bfloat16)
@@ -30,9 +32,12 @@ class TensorParallelMLP:
         """x_shards: this rank's [tokens/p, hidden] tensor (or a list, one per virtual rank)."""
         single = not isinstance(x_shards, (list, tuple))
         xs = [x_shards] if single else list(x_shards)
-        h = fused_tp.all_gather_matmul(self.comm, xs if not single else xs[0], self.w_up if not single else self.w_up[0])
+        fused = self.act is self._epilogue_act  # an activation set by hand runs as a step of its own
+        h = fused_tp.all_gather_matmul(self.comm, xs if not single else xs[0], self.w_up if not single else self.w_up[0],
+                                       activation=self.activation if fused else None)
         hs = [h] if single else h
-        hs = [self.act(t.float()).to(torch.bfloat16) for t in hs]
+        if not fused:
+            hs = [self.act(t.float()).to(torch.bfloat16) for t in hs]
         y = fused_tp.matmul_reduce_scatter(self.comm, hs if not single else hs[0], self.w_down if not single else self.w_down[0])
         return y
 

@@ -1,10 +1,10 @@
 """Fused tensor-parallel operators: tcgen05 GEMM and its NVLink collective in one sm_100a kernel.
 
-    gemm(a, b)                               -> a @ b.T                       (bf16, no communication)
-    all_gather_matmul(comm, x_shard, w)      -> all_gather_rows(x_shard) @ w.T   (column-parallel linear)
+    gemm(a, b)                               -> act(a @ b.T)                     (bf16, no communication)
+    all_gather_matmul(comm, x_shard, w)      -> act(all_gather_rows(x_shard) @ w.T)   (column-parallel linear)
     matmul_reduce_scatter(comm, h, w)        -> reduce_scatter_rows(h @ w.T)     (row-parallel linear)
 
-Weights use the nn.Linear layout [out_features, in_features].  On an all-local communicator every argument is a list
+Weights use the nn.Linear layout [out_features, in_features].  `activation` (None, "silu", "gelu") runs in the GEMM's epilogue.  On an all-local communicator every argument is a list
 with one tensor per virtual rank.
 """
 import ctypes as C
@@ -23,7 +23,10 @@ def _check(t, name):
     assert t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous(), "%s must be a contiguous CUDA bf16 tensor" % name
 
 
-def gemm(a, b, out=None):
+ACTIVATIONS = {None: 0, "none": 0, "silu": 1, "gelu": 2}
+
+
+def gemm(a, b, out=None, activation=None):
     """a [M, K] @ b[N, K].T -> [M, N] with the library's tcgen05 kernel (M % 128 == N % 256 == K % 64 == 0)."""
     _check(a, "a")
     _check(b, "b")
@@ -32,7 +35,7 @@ def gemm(a, b, out=None):
     assert b.shape[1] == K
     if out is None:
         out = torch.empty((M, N), device=a.device, dtype=torch.bfloat16)
-    L.check(L.lib().HcclB200GemmBf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, _stream()), "HcclB200GemmBf16")
+    L.check(L.lib().HcclB200GemmBf16Act(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, ACTIVATIONS[activation], _stream()), "HcclB200GemmBf16")
     return out
 
 
@@ -50,7 +53,7 @@ def _ptrs(ts):
     return (C.c_void_p * len(ts))(*[t.data_ptr() for t in ts])
 
 
-def all_gather_matmul(comm, x_shard, w, out=None):
+def all_gather_matmul(comm, x_shard, w, out=None, activation=None):
     xs, ws = _lists(comm, x_shard, w)
     for t in xs + ws:
         _check(t, "operand")
@@ -58,7 +61,8 @@ def all_gather_matmul(comm, x_shard, w, out=None):
     N = ws[0].shape[0]
     M = Ms * comm.nranks
     outs = _lists(comm, out)[0] if out is not None else [torch.empty((M, N), device=t.device, dtype=torch.bfloat16) for t in xs]
-    L.check(L.lib().HcclB200AllGatherMatmul(comm.handle, _ptrs(xs), _ptrs(ws), _ptrs(outs), M, N, K, _stream()), "HcclB200AllGatherMatmul")
+    L.check(L.lib().HcclB200AllGatherMatmulAct(comm.handle, _ptrs(xs), _ptrs(ws), _ptrs(outs), M, N, K, ACTIVATIONS[activation], _stream()),
+            "HcclB200AllGatherMatmul")
     return outs[0] if comm.nlocal == 1 else outs
 
 
