@@ -16,7 +16,8 @@ typedef HcclResult (*combine_fn)(HcclComm, const HcclB200MoeLayer *, void *const
 static collective_fn g_collective;
 static dispatch_fn g_dispatch;
 static combine_fn g_combine;
-static PyObject *s_data_ptr, *s_ctypes, *s_data;
+static PyObject *s_data_ptr, *s_ctypes, *s_data, *s_numel, *s_size, *s_dtype;
+static PyObject *g_dtypes, *g_get_device, *g_get_stream;  /* {torch / numpy dtype: HcclDataType}, current device, its current raw stream */
 
 /* address of a tensor (data_ptr()) or numpy array (ctypes.data); None is null */
 static int address(PyObject *x, void **out)
@@ -70,6 +71,86 @@ static PyObject *bind(PyObject *self, PyObject *const *a, Py_ssize_t n)
     g_combine = (combine_fn)PyLong_AsVoidPtr(a[2]);
     if (PyErr_Occurred()) return NULL;
     Py_RETURN_NONE;
+}
+
+/* setup(dtypes, get_device, get_stream): the tables and accessors that op() uses; the accessors may be None without CUDA */
+static PyObject *setup(PyObject *self, PyObject *const *a, Py_ssize_t n)
+{
+    if (n != 3 || !PyDict_Check(a[0])) { PyErr_SetString(PyExc_TypeError, "setup(dict, get_device, get_stream)"); return NULL; }
+    Py_XSETREF(g_dtypes, Py_NewRef(a[0]));
+    Py_XSETREF(g_get_device, Py_NewRef(a[1]));
+    Py_XSETREF(g_get_stream, Py_NewRef(a[2]));
+    Py_RETURN_NONE;
+}
+
+/* raw stream handle: an integer as it is, None = torch's current stream of the current device */
+static int stream_of(PyObject *x, void **out)
+{
+    if (x != Py_None) {
+        *out = PyLong_AsVoidPtr(x);
+        return *out == NULL && PyErr_Occurred() ? -1 : 0;
+    }
+    if (!g_get_stream || g_get_stream == Py_None) { PyErr_SetString(PyExc_RuntimeError, "no CUDA stream accessor"); return -1; }
+    PyObject *d = PyObject_CallNoArgs(g_get_device);
+    if (!d) return -1;
+    PyObject *s = PyObject_CallOneArg(g_get_stream, d);
+    Py_DECREF(d);
+    if (!s) return -1;
+    *out = PyLong_AsVoidPtr(s);
+    Py_DECREF(s);
+    return *out == NULL && PyErr_Occurred() ? -1 : 0;
+}
+
+/* elements and HcclDataType of a tensor or numpy array (the first one of a list) */
+static int describe(PyObject *x, uint64_t *count, int32_t *dtype)
+{
+    if (PyList_Check(x) && PyList_GET_SIZE(x)) x = PyList_GET_ITEM(x, 0);
+    else if (PyTuple_Check(x) && PyTuple_GET_SIZE(x)) x = PyTuple_GET_ITEM(x, 0);
+    PyObject *n = PyObject_CallMethodNoArgs(x, s_numel);
+    if (!n) {
+        if (!PyErr_ExceptionMatches(PyExc_AttributeError)) return -1;
+        PyErr_Clear();
+        n = PyObject_GetAttr(x, s_size);
+        if (!n) return -1;
+    }
+    *count = PyLong_AsUnsignedLongLong(n);
+    Py_DECREF(n);
+    PyObject *d = PyObject_GetAttr(x, s_dtype);
+    if (!d) return -1;
+    PyObject *code = g_dtypes ? PyDict_GetItemWithError(g_dtypes, d) : NULL;
+    if (!code) {
+        if (!PyErr_Occurred()) PyErr_SetObject(PyExc_KeyError, d);
+        Py_DECREF(d);
+        return -1;
+    }
+    Py_DECREF(d);
+    *dtype = (int32_t)PyLong_AsLong(code);
+    return PyErr_Occurred() ? -1 : 0;
+}
+
+/* op(comm, nlocal, coll, algo, nchan, op, root, send, recv, stream, by_recv, divide) -> result code: a collective whose count and
+ * type are those of the send buffer (by_recv: of the receive buffer), the count divided by `divide` */
+static PyObject *op(PyObject *self, PyObject *const *a, Py_ssize_t n)
+{
+    if (n != 12 || !g_collective) { PyErr_SetString(PyExc_TypeError, "op() takes 12 arguments, after bind()"); return NULL; }
+    HcclB200Op o;
+    memset(&o, 0, sizeof(o));
+    void *comm = PyLong_AsVoidPtr(a[0]), *stream = NULL;
+    const Py_ssize_t nlocal = PyLong_AsSsize_t(a[1]);
+    o.coll = (int32_t)PyLong_AsLong(a[2]); o.algo = (int32_t)PyLong_AsLong(a[3]); o.nchan = (int32_t)PyLong_AsLong(a[4]);
+    o.op = (int32_t)PyLong_AsLong(a[5]); o.root = (int32_t)PyLong_AsLong(a[6]);
+    const uint64_t divide = PyLong_AsUnsignedLongLong(a[11]);
+    if (PyErr_Occurred()) return NULL;
+    if (nlocal < 1 || nlocal > MAX_LOCAL || !divide) { PyErr_SetString(PyExc_ValueError, "bad number of local ranks"); return NULL; }
+    if (describe(a[10] == Py_True ? a[8] : a[7], &o.count, &o.dataType)) return NULL;
+    o.count /= divide;
+    void *send[MAX_LOCAL], *recv[MAX_LOCAL];
+    if (addresses(a[7], nlocal, send) || addresses(a[8], nlocal, recv) || stream_of(a[9], &stream)) return NULL;
+    HcclResult rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = g_collective((HcclComm)comm, &o, send, recv, (aclrtStream)stream);
+    Py_END_ALLOW_THREADS
+    return PyLong_FromLong((long)rc);
 }
 
 /* collective(comm, nlocal, coll, algo, nchan, dtype, op, root, count, send, recv, stream, tables) -> result code
@@ -145,6 +226,8 @@ static PyObject *moe_combine(PyObject *self, PyObject *const *a, Py_ssize_t n)
 }
 
 static PyMethodDef methods[] = {{"bind", (PyCFunction)(void (*)(void))bind, METH_FASTCALL, NULL},
+                                {"setup", (PyCFunction)(void (*)(void))setup, METH_FASTCALL, NULL},
+                                {"op", (PyCFunction)(void (*)(void))op, METH_FASTCALL, NULL},
                                 {"moe_dispatch", (PyCFunction)(void (*)(void))moe_dispatch, METH_FASTCALL, NULL},
                                 {"moe_combine", (PyCFunction)(void (*)(void))moe_combine, METH_FASTCALL, NULL},
                                 {"collective", (PyCFunction)(void (*)(void))collective, METH_FASTCALL, NULL},
@@ -156,5 +239,8 @@ PyMODINIT_FUNC PyInit__fastcall(void)
     s_data_ptr = PyUnicode_InternFromString("data_ptr");
     s_ctypes = PyUnicode_InternFromString("ctypes");
     s_data = PyUnicode_InternFromString("data");
+    s_numel = PyUnicode_InternFromString("numel");
+    s_size = PyUnicode_InternFromString("size");
+    s_dtype = PyUnicode_InternFromString("dtype");
     return PyModule_Create(&module);
 }

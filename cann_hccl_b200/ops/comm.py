@@ -9,7 +9,7 @@ import json
 import numpy as np
 
 from .. import _lib as L
-from ..utils.dtypes import data_ptr, hccl_dtype, numel
+from ..utils.dtypes import data_ptr, dtype_table, hccl_dtype, numel
 
 
 _U64 = np.dtype(np.uint64)
@@ -24,6 +24,7 @@ def _u64(a):
 class Communicator:
     def __init__(self, handle, device):
         self._h = C.c_void_p(handle)
+        self._hv = handle or 0  # the same as an integer, for the native call path
         self.device = bool(device)
         lib = L.lib()
         n, r, nl = C.c_uint32(), C.c_uint32(), C.c_uint32()
@@ -32,6 +33,7 @@ class Communicator:
         L.check(lib.HcclB200GetLocalRankNum(self._h, C.byref(nl)), "HcclB200GetLocalRankNum")
         self.nranks, self.rank, self.nlocal = n.value, r.value, nl.value
         self._keep = []
+        _fast_setup(self.device)
 
     # ------------------------------------------------------------------ creation
     @staticmethod
@@ -100,12 +102,12 @@ class Communicator:
 
     def destroy(self):
         if not getattr(self, "_owned", True):
-            self._h = C.c_void_p()
+            self._h, self._hv = C.c_void_p(), 0
             return L.SUCCESS
         if self._h and self._h.value:
             code = L.lib().HcclCommDestroy(self._h)
             if code == L.SUCCESS:
-                self._h = C.c_void_p()
+                self._h, self._hv = C.c_void_p(), 0
             return code
         return L.SUCCESS
 
@@ -138,7 +140,7 @@ class Communicator:
             st = _raw_stream()
         else:
             st = stream if isinstance(stream, int) else stream.cuda_stream
-        code = L.fast.collective(self._h.value or 0, self.nlocal, coll, algo, nchan, dtype, op, root, int(count), send, recv, st, tables)
+        code = L.fast.collective(self._hv, self.nlocal, coll, algo, nchan, dtype, op, root, int(count), send, recv, st, tables)
         if code:
             L.check(code, "HcclB200Collective(%d)" % coll)
 
@@ -160,17 +162,29 @@ class Communicator:
     def _first(self, x):
         return x[0] if isinstance(x, (list, tuple)) else x
 
+    def _op(self, coll, send, recv, op, root, algo, nchan, stream, by_recv=False, divide=1):
+        """A collective described by its buffers alone: count and type come from the first of them."""
+        if not self.device:
+            stream = 0
+        elif stream is not None and not isinstance(stream, int):
+            stream = stream.cuda_stream
+        try:
+            code = L.fast.op(self._hv, self.nlocal, coll, algo, nchan, op, root, send, recv, stream, by_recv, divide)
+        except KeyError:  # torch tensors on the host transport, torch imported after the communicator was made
+            if not _fast_torch_types():
+                raise
+            code = L.fast.op(self._hv, self.nlocal, coll, algo, nchan, op, root, send, recv, stream, by_recv, divide)
+        if code:
+            L.check(code, "HcclB200Collective(%d)" % coll)
+
     def all_reduce(self, send, recv, op=L.SUM, algo=L.ALGO_AUTO, nchan=0, stream=None):
-        f = self._first(send)
-        self.collective(L.ALLREDUCE, send, recv, numel(f), hccl_dtype(f), op=op, algo=algo, nchan=nchan, stream=stream)
+        self._op(L.ALLREDUCE, send, recv, op, 0, algo, nchan, stream)
 
     def broadcast(self, buf, root, algo=L.ALGO_AUTO, nchan=0, stream=None):
-        f = self._first(buf)
-        self.collective(L.BROADCAST, buf, buf, numel(f), hccl_dtype(f), root=root, algo=algo, nchan=nchan, stream=stream)
+        self._op(L.BROADCAST, buf, buf, L.SUM, root, algo, nchan, stream)
 
     def reduce_scatter(self, send, recv, op=L.SUM, algo=L.ALGO_AUTO, nchan=0, stream=None):
-        f = self._first(recv)
-        self.collective(L.REDUCE_SCATTER, send, recv, numel(f), hccl_dtype(f), op=op, algo=algo, nchan=nchan, stream=stream)
+        self._op(L.REDUCE_SCATTER, send, recv, op, 0, algo, nchan, stream, True)
 
     def reduce_scatter_v(self, send, recv, counts, displs, op=L.SUM, algo=L.ALGO_AUTO, nchan=0, stream=None):
         f = self._first(send)
@@ -178,8 +192,7 @@ class Communicator:
                         displs=displs, stream=stream)
 
     def all_gather(self, send, recv, algo=L.ALGO_AUTO, nchan=0, stream=None):
-        f = self._first(send)
-        self.collective(L.ALLGATHER, send, recv, numel(f), hccl_dtype(f), algo=algo, nchan=nchan, stream=stream)
+        self._op(L.ALLGATHER, send, recv, L.SUM, 0, algo, nchan, stream)
 
     def all_gather_v(self, send, recv, counts, displs, algo=L.ALGO_AUTO, nchan=0, stream=None):
         f = self._first(recv)
@@ -187,20 +200,16 @@ class Communicator:
                         stream=stream)
 
     def reduce(self, send, recv, root, op=L.SUM, algo=L.ALGO_AUTO, nchan=0, stream=None):
-        f = self._first(send)
-        self.collective(L.REDUCE, send, recv, numel(f), hccl_dtype(f), op=op, root=root, algo=algo, nchan=nchan, stream=stream)
+        self._op(L.REDUCE, send, recv, op, root, algo, nchan, stream)
 
     def scatter(self, send, recv, root, algo=L.ALGO_AUTO, nchan=0, stream=None):
-        f = self._first(recv)
-        self.collective(L.SCATTER, send, recv, numel(f), hccl_dtype(f), root=root, algo=algo, nchan=nchan, stream=stream)
+        self._op(L.SCATTER, send, recv, L.SUM, root, algo, nchan, stream, True)
 
     def gather(self, send, recv, root, algo=L.ALGO_AUTO, nchan=0, stream=None):
-        f = self._first(send)
-        self.collective(L.GATHER, send, recv, numel(f), hccl_dtype(f), root=root, algo=algo, nchan=nchan, stream=stream)
+        self._op(L.GATHER, send, recv, L.SUM, root, algo, nchan, stream)
 
     def all_to_all(self, send, recv, algo=L.ALGO_AUTO, nchan=0, stream=None):
-        f = self._first(send)
-        self.collective(L.ALLTOALL, send, recv, numel(f) // self.nranks, hccl_dtype(f), algo=algo, nchan=nchan, stream=stream)
+        self._op(L.ALLTOALL, send, recv, L.SUM, 0, algo, nchan, stream, False, self.nranks)
 
     def all_to_all_v(self, send, send_counts, sdispls, recv, recv_counts, rdispls, algo=L.ALGO_AUTO, nchan=0, stream=None):
         f = self._first(send)
@@ -437,6 +446,32 @@ class Communicator:
 
 
 _RAW = _DEV = None
+_fast_ready = 0
+
+
+def _fast_setup(device):
+    """Hands the native call path its type table and, on the device transport, torch's stream accessors."""
+    global _fast_ready
+    want = 2 if device else 1
+    if _fast_ready >= want:
+        return
+    if device:
+        _raw_stream()
+        get_dev, get = (_DEV, _RAW) if _RAW else (lambda: None, lambda _: _raw_stream())
+        L.fast.setup(dtype_table(True), get_dev, get)
+    else:
+        L.fast.setup(dtype_table(False), None, None)
+    _fast_ready = want
+
+
+def _fast_torch_types():
+    """Adds the torch dtypes to a table made without them; False when they are there already."""
+    global _fast_ready
+    if _fast_ready != 1:
+        return False
+    L.fast.setup(dtype_table(True), None, None)
+    _fast_ready = 1.5
+    return True
 
 
 def _raw_stream():

@@ -22,6 +22,11 @@ def _torch_map():
 _TORCH = None
 
 
+def dtype_table(torch_too):
+    """{numpy dtype: HcclDataType}, with the torch dtypes where buffers are torch tensors."""
+    return {**_NP, **_torch_map()} if torch_too else dict(_NP)
+
+
 def hccl_dtype(x):
     """HcclDataType of a numpy array or torch tensor."""
     global _TORCH
