@@ -37,14 +37,14 @@ HcclResult Communicator::run_direct(const OpRequest &rq)
         r.p = p;
         if (rq.coll == COLL_ALLREDUCE || rq.coll == COLL_REDUCE) {
             r.njobs = 1;
-            r.off[0] = 0; r.count[0] = n; r.mask[0] = rq.coll == COLL_ALLREDUCE ? all : 1u << rq.root;
+            r.job[0].off = 0; r.job[0].count = n; r.job[0].mask = rq.coll == COLL_ALLREDUCE ? all : 1u << rq.root;
         } else {
             r.njobs = p;
             for (int j = 0; j < p; ++j) {
                 const bool v = rq.coll == COLL_REDUCE_SCATTER_V;
-                r.off[j] = (v ? rq.displs[j] : (uint64_t)j * n) * es;
-                r.count[j] = v ? rq.counts[j] : n;
-                r.mask[j] = 1u << j;
+                r.job[j].off = (v ? rq.displs[j] : (uint64_t)j * n) * es;
+                r.job[j].count = v ? rq.counts[j] : n;
+                r.job[j].mask = 1u << j;
             }
         }
         return launch_local_reduce(r, rq.dtype, rq.redop, rq.stream);
@@ -53,7 +53,7 @@ HcclResult Communicator::run_direct(const OpRequest &rq)
     LocalCopy c;
     c.njobs = 0;
     for (int q = 0; q < p; ++q) c.out[q] = (uint8_t *)rq.out[q];
-    // ranks of `mask` that already hold the block where it belongs (in-place forms) drop out; destinations whose 16-byte
+    // ranks of `mask` that already hold the block where it belongs (in-place forms) drop out; destinations whose 32-byte
     // alignments differ become jobs of their own
     auto add = [&](const void *src, uint64_t doff, uint64_t bytes, uint32_t mask) {
         if (!bytes) return;
@@ -63,7 +63,7 @@ HcclResult Communicator::run_direct(const OpRequest &rq)
             const int first = __builtin_ctz(mask);
             uint32_t same = 0;
             for (int d = first; d < p; ++d)
-                if (((mask >> d) & 1u) && ((((uintptr_t)c.out[d]) ^ ((uintptr_t)c.out[first])) & 15) == 0) same |= 1u << d;
+                if (((mask >> d) & 1u) && ((((uintptr_t)c.out[d]) ^ ((uintptr_t)c.out[first])) & 31) == 0) same |= 1u << d;
             c.job[c.njobs++] = LocalCopyJob{(const uint8_t *)src, doff, bytes, 0, same};
             mask &= ~same;
         }

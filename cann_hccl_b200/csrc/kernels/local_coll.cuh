@@ -6,7 +6,7 @@
 
 namespace hcclb {
 
-constexpr int kLocalThreads = 256;
+constexpr int kLocalThreads = 128;
 
 // 16 bytes at v0 + s (0 < s < 16), v0 and v1 being the two aligned vectors that hold them.  s is uniform in a job.
 __device__ __forceinline__ uint4 merge16(uint4 v0, uint4 v1, uint32_t s)
@@ -30,100 +30,118 @@ __device__ __forceinline__ uint4 ld_shifted(const uint8_t *a)
     return s ? merge16(b[0], b[1], s) : b[0];
 }
 
-// One tile of a job: U vectors of every source in flight per thread.  SHIFT: some source is not aligned like the outputs.
-template <class T, int OP, int NP, int U, bool SHIFT>
-__device__ __forceinline__ void local_reduce_tile(const uint8_t *const (&in)[kMaxRanks], uint8_t *const (&out)[kMaxRanks], uint32_t mask, uint64_t soff,
-                                                  uint64_t doff, int p, uint64_t v0, uint64_t v1)
+// A vector is one load per source: 32 bytes where every address allows it, else 16.
+template <int VB> union Vec;
+template <> union Vec<16> { uint4 u; uint32_t w[4]; };
+template <> union Vec<32> { uint4 u[2]; uint32_t w[8]; };
+__device__ __forceinline__ Vec<16> ld_vec(const uint8_t *p, Vec<16> *) { Vec<16> v; v.u = ld_stream((const uint4 *)p); return v; }
+__device__ __forceinline__ Vec<32> ld_vec(const uint8_t *p, Vec<32> *)
+{
+    Vec<32> v;
+    asm volatile("ld.global.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v.w[0]), "=r"(v.w[1]), "=r"(v.w[2]), "=r"(v.w[3]), "=r"(v.w[4]), "=r"(v.w[5]), "=r"(v.w[6]), "=r"(v.w[7]) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_vec(uint8_t *p, const Vec<16> &v) { *(uint4 *)p = v.u; }
+__device__ __forceinline__ void st_vec(uint8_t *p, const Vec<32> &v)
+{
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 ::"l"(p), "r"(v.w[0]), "r"(v.w[1]), "r"(v.w[2]), "r"(v.w[3]), "r"(v.w[4]), "r"(v.w[5]), "r"(v.w[6]), "r"(v.w[7]) : "memory");
+}
+
+// Vectors per thread of a full tile: 128 bytes of loads in flight per thread for two sources, 128 to 256 for more.
+template <int NP, int VB> constexpr int kReduceVecs = NP == 2 ? 64 / VB : (NP == 4 ? 32 / VB : 1);
+
+// One tile of a job.  SHIFT: some source is not aligned like the outputs.
+template <class T, int OP, int NP, int VB, int U, bool SHIFT>
+__device__ __forceinline__ void local_reduce_tile(const LocalReduce &a, const LocalReduceJob &j, uint32_t tile)
 {
     using N = DNum<T>;
     using Acc = typename N::Acc;
-    constexpr int E = 16 / sizeof(T);
-    for (uint64_t i = v0 + threadIdx.x; i < v1; i += (uint64_t)U * kLocalThreads) {
+    constexpr int E = VB / sizeof(T);
+    union Elems { Vec<VB> v; T e[E]; __device__ Elems() {} };
+    const uint64_t first = (uint64_t)tile * a.tile_vecs + threadIdx.x, soff = j.off + j.head * sizeof(T), doff = j.head * sizeof(T);
+    const uint64_t end = min(j.nvec, (uint64_t)(tile + 1) * a.tile_vecs);
+#pragma unroll 1
+    for (uint64_t i = first; i < end; i += (uint64_t)U * kLocalThreads) {
         Acc acc[U][E];
-        for (int q0 = 0; q0 < p; q0 += NP) {
-            uint4 x[U][NP];
+#pragma unroll 1
+        for (int q0 = 0; q0 < a.p; q0 += NP) {
+            Elems x[U][NP];
 #pragma unroll
             for (int u = 0; u < U; ++u)
 #pragma unroll
                 for (int q = 0; q < NP; ++q) {
                     const uint64_t v = i + (uint64_t)u * kLocalThreads;
-                    if (q0 + q < p && v < v1) {
-                        const uint8_t *a = in[q0 + q] + soff + (v << 4);
-                        x[u][q] = SHIFT ? ld_shifted(a) : ld_stream((const uint4 *)a);
+                    if (q0 + q < a.p && v < end) {
+                        const uint8_t *s = a.in[q0 + q] + soff + v * VB;
+                        if constexpr (SHIFT) x[u][q].v.u = ld_shifted(s);
+                        else x[u][q].v = ld_vec(s, (Vec<VB> *)nullptr);
                     }
                 }
 #pragma unroll
             for (int u = 0; u < U; ++u)
 #pragma unroll
                 for (int q = 0; q < NP; ++q)
-                    if (q0 + q < p) {
-                        Pack16<T> t;
-                        t.u = x[u][q];
+                    if (q0 + q < a.p) {
 #pragma unroll
-                        for (int k = 0; k < E; ++k) acc[u][k] = q == 0 && q0 == 0 ? N::up(t.e[k]) : red_op<OP>(acc[u][k], N::up(t.e[k]));
+                        for (int k = 0; k < E; ++k) acc[u][k] = q == 0 && q0 == 0 ? N::up(x[u][q].e[k]) : red_op<OP>(acc[u][k], N::up(x[u][q].e[k]));
                     }
             if (NP < 8) break;  // the launcher takes the batch of eight for five and more ranks
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const uint64_t v = i + (uint64_t)u * kLocalThreads;
-            if (v < v1) {
-                Pack16<T> z;
+            if (v < end) {
+                Elems z;
 #pragma unroll
                 for (int k = 0; k < E; ++k) z.e[k] = N::down(acc[u][k]);
-#pragma unroll
-                for (int d = 0; d < kMaxRanks; ++d)
-                    if ((mask >> d) & 1u) *(uint4 *)(out[d] + doff + (v << 4)) = z.u;
+                for (uint32_t m = j.mask; m; m &= m - 1) st_vec(a.out[__ffs(m) - 1] + doff + v * VB, z.v);
             }
         }
     }
 }
 
-template <class T, int OP, int NP>
+template <class T, int OP, int NP, int VB>
 __global__ void __launch_bounds__(kLocalThreads) local_reduce_kernel(const __grid_constant__ LocalReduce a)
 {
     using N = DNum<T>;
     using Acc = typename N::Acc;
-    constexpr int E = 16 / sizeof(T), U = NP == 2 ? 4 : (NP == 4 ? 2 : 1);
+    constexpr int E = VB / sizeof(T);
     pdl_trigger();
-    int j = 0;
-    while (blockIdx.x >= a.tile0[j + 1]) ++j;  // the launcher's table ends with the grid's size
-    const uint64_t n = a.count[j], soff = a.off[j];
-    const uint32_t mask = a.mask[j], tile = blockIdx.x - a.tile0[j];
-    // vectors are laid over the outputs' 16-byte granules; the elements before the first and after the last go one by one
-    const uint8_t *d0 = a.out[__ffs(mask) - 1];
-    uint32_t differ = 0, shift = 0;
-#pragma unroll
-    for (int d = 0; d < kMaxRanks; ++d)
-        if ((mask >> d) & 1u) differ |= (uint32_t)((uintptr_t)a.out[d] ^ (uintptr_t)d0) & 15;
-    uint64_t head = ((16 - ((uintptr_t)d0 & 15)) & 15) / sizeof(T);
-    if (head > n || differ) head = n;
-    const uint64_t nvec = (n - head) / E, hb = head * sizeof(T);
-    for (int q = 0; q < a.p; ++q) shift |= (uint32_t)((uintptr_t)a.in[q] + soff + hb) & 15;
+    int ji = 0;
+    if (a.uniform) ji = blockIdx.x / a.uniform;
+    else
+        while (ji + 1 < a.njobs && blockIdx.x >= a.job[ji + 1].tile0) ++ji;
+    const LocalReduceJob &j = a.job[ji];
+    const uint32_t tile = blockIdx.x - j.tile0;
     pdl_wait();
-    const uint64_t v0 = (uint64_t)tile * a.tile_vecs, v1 = v0 + a.tile_vecs < nvec ? v0 + a.tile_vecs : nvec;
-    if (v0 < nvec) {
-        if (!shift) local_reduce_tile<T, OP, NP, U, false>(a.in, a.out, mask, soff + hb, hb, a.p, v0, v1);
-        else local_reduce_tile<T, OP, NP, 1, true>(a.in, a.out, mask, soff + hb, hb, a.p, v0, v1);
+    if (j.layout != LOCAL_SCALAR && (uint64_t)tile * a.tile_vecs < j.nvec) {
+        if (VB == 32 || j.layout == LOCAL_ALIGNED) local_reduce_tile<T, OP, NP, VB, kReduceVecs<NP, VB>, false>(a, j, tile);
+        else if constexpr (VB == 16) local_reduce_tile<T, OP, NP, 16, 1, true>(a, j, tile);
+        return;
     }
-    // leftovers: at most a vector at either end, or everything when the outputs do not share an alignment
-    const uint64_t left = n - nvec * E, step = differ ? (uint64_t)(a.tile0[j + 1] - a.tile0[j]) * kLocalThreads : kLocalThreads;
-    if (tile != 0 && !differ) return;
-    for (uint64_t l = (uint64_t)(differ ? tile : 0) * kLocalThreads + threadIdx.x; l < left; l += step) {
-        const uint64_t e = l < head ? l : nvec * E + l;
-        Acc acc = N::up(((const T *)(a.in[0] + soff))[e]);
-        for (int q = 1; q < a.p; ++q) acc = red_op<OP>(acc, N::up(((const T *)(a.in[q] + soff))[e]));
+    // one by one: what lies outside the vectors (a tile of its own), or everything when the outputs do not share an alignment
+    const bool scalar = j.layout == LOCAL_SCALAR;
+    const uint64_t vecs = scalar ? 0 : j.nvec, left = j.count - vecs * E;
+    const uint64_t l0 = scalar ? (uint64_t)tile * a.tile_vecs * E : 0, l1 = scalar ? min(left, l0 + (uint64_t)a.tile_vecs * E) : left;
+    for (uint64_t l = l0 + threadIdx.x; l < l1; l += kLocalThreads) {
+        const uint64_t e = l < j.head ? l : vecs * E + l;
+        Acc acc = N::up(((const T *)(a.in[0] + j.off))[e]);
+        for (int q = 1; q < a.p; ++q) acc = red_op<OP>(acc, N::up(((const T *)(a.in[q] + j.off))[e]));
         const T r = N::down(acc);
-        for (int d = 0; d < kMaxRanks; ++d)
-            if ((mask >> d) & 1u) ((T *)a.out[d])[e] = r;
+        for (uint32_t m = j.mask; m; m &= m - 1) ((T *)a.out[__ffs(m) - 1])[e] = r;
     }
 }
 
-// Defines local_kernel_<name>(op, p): the reduction kernel for element type T.
-#define HCCLB_LOCAL_BATCH(T, OP) \
-    (p <= 2 ? (const void *)local_reduce_kernel<T, OP, 2> : p <= 4 ? (const void *)local_reduce_kernel<T, OP, 4> : (const void *)local_reduce_kernel<T, OP, 8>)
+// Defines local_kernel_<name>(op, p, wide): the reduction kernel for element type T; wide: vectors of 32 bytes.
+#define HCCLB_LOCAL_BATCH(T, OP)                                                                                                            \
+    (wide ? (p <= 2 ? (const void *)local_reduce_kernel<T, OP, 2, 32> : p <= 4 ? (const void *)local_reduce_kernel<T, OP, 4, 32>           \
+                                                                               : (const void *)local_reduce_kernel<T, OP, 8, 32>)          \
+          : (p <= 2 ? (const void *)local_reduce_kernel<T, OP, 2, 16> : p <= 4 ? (const void *)local_reduce_kernel<T, OP, 4, 16>           \
+                                                                               : (const void *)local_reduce_kernel<T, OP, 8, 16>))
 #define HCCLB_INSTANTIATE_LOCAL(T, name)                                              \
-    const void *local_kernel_##name(int op, int p)                                    \
+    const void *local_kernel_##name(int op, int p, bool wide)                         \
     {                                                                                 \
         switch (op) {                                                                 \
             case HCCL_REDUCE_SUM: return HCCLB_LOCAL_BATCH(T, HCCL_REDUCE_SUM);       \

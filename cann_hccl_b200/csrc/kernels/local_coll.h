@@ -5,9 +5,10 @@
 //
 // Bound: HBM for messages beyond L2, launch and one memory round trip below.  Measured on a B200 against the staged kernels
 // (push, reduce and copy-out through staging buffers, CTAs of all ranks resident together): AllReduce of 64 MiB fp32 over
-// eight ranks 655 -> 164 us (6.56 TB/s), ReduceScatter of 4 MiB bf16 blocks over eight ranks 286 -> 55 us, AlltoAllV of 1024
-// rows of 7168 bf16 from each of eight ranks 138 -> 37 us, AllGather of 1 MiB over four ranks 31 -> 8.5 us, the copy of a
-// single rank's 64 MiB 28.8 -> 21.8 us (6.2 TB/s).
+// eight ranks 655 -> 159 us (6.8 TB/s), ReduceScatter of 4 MiB bf16 blocks over eight ranks 286 -> 46 us (6.6 TB/s), AlltoAllV
+// of 1024 rows of 7168 bf16 from each of eight ranks 138 -> 36 us, the copy of a single rank's 64 MiB 28.8 -> 21.4 us.
+// What the last steps gave (ReduceScatter case): how a job lies over vectors worked out by the launcher instead of by every
+// CTA, 55 -> 50 us; 32-byte instead of 16-byte vectors, 50 -> 46 us.
 #pragma once
 #include "algo/plan.h"
 
@@ -27,15 +28,22 @@ struct LocalCopy {
     int njobs;
     LocalCopyJob job[kLocalMaxJobs];
 };
-// Job j: out[d] (d in mask[j]) = reduction over the p ranks, in rank order, of count[j] elements at in[q] + off[j].
+// Job: out[d] (d in mask) = reduction over the p ranks, in rank order, of `count` elements at in[q] + off.  The launcher fills
+// in how the job is laid over vectors, so that a CTA loads a few words and starts.
+enum LocalLayout : uint32_t { LOCAL_ALIGNED = 0, LOCAL_SHIFTED = 1, LOCAL_SCALAR = 2 };
+struct LocalReduceJob {
+    uint64_t off, count;
+    uint32_t mask, layout;
+    uint64_t nvec;       // vectors of the outputs
+    uint32_t head;       // elements before the first vector
+    uint32_t tile0;      // first tile; the job's last tile holds the elements outside the vectors when there are any
+};
 struct LocalReduce {
     const uint8_t *in[kMaxRanks];
     uint8_t *out[kMaxRanks];
-    uint64_t off[kMaxRanks], count[kMaxRanks];
-    uint32_t tile0[kMaxRanks + 1];  // first tile of a job (filled by the launcher)
-    uint32_t mask[kMaxRanks];
+    LocalReduceJob job[kMaxRanks];
     int p, njobs;
-    uint32_t tile_vecs;
+    uint32_t tile_vecs, uniform;  // uniform: tiles per job when all jobs have the same number, else 0
 };
 
 // Both take and change the caller's description (tile tables).
