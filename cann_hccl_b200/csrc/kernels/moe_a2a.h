@@ -14,18 +14,18 @@ HcclResult moe_combine(void *const *y_peers, const int32_t *topk_idx, const floa
                        int hidden, int n_experts, int p, int me, int pairwise, void *out, int64_t capacity_rows, void *stream);
 
 // ---- all ranks in this process on one GPU (kernels/moe_local.cu)
-constexpr int kMoeLocalMaxExperts = 8192;  // one shared-memory counter each
+constexpr int kMoeLocalMaxExperts = 4096;  // two shared-memory words each
 struct MoeLocalLayer {
     int64_t tokens, capacity;  // tokens of a rank; rows of a receive buffer
     int p, topk, hidden, n_experts;
     int32_t *const *pos, *const *dst_row, *const *expert_offsets, *const *recv_rows, *const *overflow;  // [p] device pointers
     int32_t *scratch;          // moe_local_scratch_words() words, zero before the first call
 };
-// The count kernel cuts a rank's pairs into chunks: one CTA numbers a chunk in shared memory.  At most 32 chunks: the CTA that
+// The count kernel cuts a rank's pairs into chunks: one CTA numbers a chunk in shared memory.  At most 64 chunks: the CTA that
 // turns the histograms into row bases reads all of them.
 inline void moe_local_chunks(int64_t npairs, int *chunk, int *nchunk)
 {
-    const int64_t c = std::max<int64_t>(1024, (npairs + 31) / 32);
+    const int64_t c = std::max<int64_t>(1024, (npairs + 63) / 64);
     *chunk = (int)c;
     *nchunk = (int)std::max<int64_t>(1, (npairs + c - 1) / c);
 }

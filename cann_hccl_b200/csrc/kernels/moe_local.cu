@@ -7,7 +7,12 @@
 //             receive rows: tokens x (1 + k) rows of traffic, the least the exchange can do;
 //   combine   the same split over the output rows: eight expert rows in flight per thread, fp32 sum in k order, one rounding.
 //
-// Bound: HBM for prefill batches, launches and latency for decode batches.
+// A decode batch (8192 pairs and fewer over all ranks) has its rows from ONE CTA that counts in shared memory and registers.
+//
+// Bound: HBM for prefill batches (8192 tokens x 7168, top 8, one rank: dispatch 165 us at 6.4 TB/s, combine 156 us at 6.8 TB/s,
+// whole exchange 338 us, 468 us with a row read per expert, a launch per rank and step, and barriers), launches and L2 for
+// decode batches (128 tokens on each of four ranks: 26 us, 301 us before).  Dispatch with 16-byte instead of 32-byte vectors:
+// 171 us; counting a decode batch with the prefill kernel: 9 us instead of 5.6 us.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <algorithm>
@@ -20,7 +25,46 @@ namespace hcclb {
 
 namespace {
 
-constexpr int kCountThreads = 512, kRowThreads = 256, kRowBatch = 8;
+constexpr int kCountThreads = 1024, kScanRegs = 16, kRowsRegs = 8, kDispatchThreads = 128, kRowThreads = 256, kRowBatch = 8;
+
+struct alignas(32) Row32 { uint32_t w[8]; };
+__device__ __forceinline__ uint4 ld_row(const uint4 *p) { return *p; }
+__device__ __forceinline__ void st_row(uint4 *p, const uint4 &v) { *p = v; }
+__device__ __forceinline__ Row32 ld_row(const Row32 *p)
+{
+    Row32 v;
+    asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v.w[0]), "=r"(v.w[1]), "=r"(v.w[2]), "=r"(v.w[3]), "=r"(v.w[4]), "=r"(v.w[5]), "=r"(v.w[6]), "=r"(v.w[7]) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_row(Row32 *p, const Row32 &v)
+{
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 ::"l"(p), "r"(v.w[0]), "r"(v.w[1]), "r"(v.w[2]), "r"(v.w[3]), "r"(v.w[4]), "r"(v.w[5]), "r"(v.w[6]), "r"(v.w[7]) : "memory");
+}
+
+// Exclusive prefix of t over the CTA's kCountThreads threads; *all becomes the sum.  Two barriers.
+__device__ __forceinline__ int cta_prefix(int t, int *s_warp, int *all)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto inclusive = [&](int v) {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int w = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += w;
+        }
+        return v;
+    };
+    const int v = inclusive(t);
+    if (lane == 31) s_warp[warp] = v;
+    __syncthreads();
+    const int sum = s_warp[lane], w = inclusive(sum);
+    static_assert(kCountThreads == 1024, "one lane per warp of the CTA");
+    const int before = __shfl_sync(0xffffffffu, w - sum, warp);
+    *all = __shfl_sync(0xffffffffu, w, 31);
+    __syncthreads();
+    return before + v - t;
+}
 
 struct MoeTables {
     const __nv_bfloat16 *x[kMaxRanks];
@@ -38,7 +82,7 @@ struct MoeTables {
 // grid (chunks, ranks)
 __global__ void __launch_bounds__(kCountThreads) moe_local_count_kernel(const __grid_constant__ MoeTables a)
 {
-    extern __shared__ int32_t sh[];  // [experts]
+    extern __shared__ int32_t sh[];  // [experts + 1], then [parts][experts]
     __shared__ int s_last;
     pdl_trigger();
     const int E = a.n_experts, r = blockIdx.y;
@@ -52,102 +96,178 @@ __global__ void __launch_bounds__(kCountThreads) moe_local_count_kernel(const __
     }
     __syncthreads();
     for (int e = threadIdx.x; e < E; e += kCountThreads) a.hist[((int64_t)r * a.nchunk + blockIdx.x) * E + e] = sh[e];
-    __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(a.arrived, 1u) == gridDim.x * gridDim.y - 1;
+    if (threadIdx.x == 0) {  // the barrier puts the CTA's histogram before this thread's fence
+        __threadfence();
+        s_last = atomicAdd(a.arrived, 1u) == gridDim.x * gridDim.y - 1;
+        __threadfence();
+    }
     __syncthreads();
     if (!s_last) return;
-    __threadfence();
-    // rows of an owner are grouped [local expert][source rank][chunk]
-    const int groups = a.p * a.nchunk, El = E / a.p;
-    for (int e = threadIdx.x; e < E; e += kCountThreads) {
+    // Rows of an owner are grouped [local expert][source rank][chunk].  `parts` threads share an expert's groups, so that their
+    // loads are one round trip (a few registers each) where the experts leave threads over.
+    const int groups = a.p * a.nchunk, El = E / a.p, parts = max(1, kCountThreads / E), per = (groups + parts - 1) / parts;
+    int32_t *sub = sh + E + 1;  // [part][expert]: pairs of the part, then its first row within the expert
+    __shared__ int s_warp[kCountThreads / 32];
+    const bool once = parts * E <= kCountThreads && per <= kScanRegs;  // a thread's groups stay in its registers
+    int n[kScanRegs];
+    for (int i = threadIdx.x; i < parts * E; i += kCountThreads) {
+        const int part = i / E, e = i - part * E, g0 = part * per, g1 = min(groups, g0 + per);
         int t = 0;
-#pragma unroll 8
-        for (int g = 0; g < groups; ++g) t += __ldcg(a.hist + (int64_t)g * E + e);
-        sh[e] = t;
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {  // exclusive prefix over all experts
-        int carry = 0;
-        for (int e0 = 0; e0 < E; e0 += 32) {
-            const int e = e0 + threadIdx.x, t = e < E ? sh[e] : 0;
-            int v = t;
+        for (int gb = g0; gb < g1; gb += kScanRegs) {
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int w = __shfl_up_sync(0xffffffffu, v, o);
-                if ((int)threadIdx.x >= o) v += w;
-            }
-            if (e < E) sh[e] = carry + v - t;
-            carry += __shfl_sync(0xffffffffu, v, 31);
+            for (int k = 0; k < kScanRegs; ++k) n[k] = gb + k < g1 ? __ldcg(a.hist + (int64_t)(gb + k) * E + e) : 0;
+#pragma unroll
+            for (int k = 0; k < kScanRegs; ++k) t += n[k];
         }
-        if (threadIdx.x == 0) { sh[E] = carry; *a.arrived = 0; }
+        sub[i] = t;
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < E; e += kCountThreads) {
-        const int q = e / El, first = sh[q * El];
-        int row = sh[e] - first;
-        a.expert_offsets[q][e - q * El] = row;
-        if (e == q * El + El - 1) {
-            const int total = sh[e + 1] - first;
-            a.expert_offsets[q][El] = total;
-            *a.recv_rows[q] = total;
-            if (total > a.capacity) *a.overflow[q] = 1;
+    // exclusive prefix over all experts, kCountThreads of them at a time
+    int carry = 0;
+    for (int e0 = 0; e0 < E; e0 += kCountThreads) {
+        const int e = e0 + threadIdx.x;
+        int t = 0;
+        if (e < E)
+            for (int q = 0; q < parts; ++q) { const int v = sub[q * E + e]; sub[q * E + e] = t; t += v; }
+        int all;
+        const int before = cta_prefix(t, s_warp, &all);
+        if (e < E) sh[e] = carry + before;
+        carry += all;
+    }
+    if (threadIdx.x == 0) { sh[E] = carry; *a.arrived = 0; }
+    __syncthreads();
+    for (int i = threadIdx.x; i < parts * E; i += kCountThreads) {
+        const int part = i / E, e = i - part * E, q = e / El, first = sh[q * El], g0 = part * per, g1 = min(groups, g0 + per);
+        int row = sh[e] - first + sub[i];
+        for (int gb = g0; gb < g1; gb += kScanRegs) {
+            if (!once)
+#pragma unroll
+                for (int k = 0; k < kScanRegs; ++k) n[k] = gb + k < g1 ? __ldcg(a.hist + (int64_t)(gb + k) * E + e) : 0;
+#pragma unroll
+            for (int k = 0; k < kScanRegs; ++k)
+                if (gb + k < g1) {
+                    a.hist[(int64_t)(gb + k) * E + e] = row;
+                    row += n[k];
+                }
         }
-#pragma unroll 8
-        for (int g = 0; g < groups; ++g) {
-            int32_t *h = a.hist + (int64_t)g * E + e;
-            const int n = __ldcg(h);
-            *h = row;
-            row += n;
+        if (part == 0) {
+            a.expert_offsets[q][e - q * El] = sh[e] - first;
+            if (e == q * El + El - 1) {
+                const int total = sh[e + 1] - first;
+                a.expert_offsets[q][El] = total;
+                *a.recv_rows[q] = total;
+                if (total > a.capacity) *a.overflow[q] = 1;
+            }
         }
     }
 }
 
-// grid (tokens x segments, ranks)
-__global__ void __launch_bounds__(kRowThreads) moe_local_dispatch_kernel(const __grid_constant__ MoeTables a)
+// Few pairs (a decode batch): one CTA numbers the pairs of all ranks and knows their rows without a trip through global memory
+// (no histogram, no fence, no arrival).  A thread keeps its pairs in registers.  Dynamic shared memory: [rank][expert] counters,
+// then their first rows; [experts + 1] first row of an expert over all owners.
+__global__ void __launch_bounds__(kCountThreads) moe_local_rows_kernel(const __grid_constant__ MoeTables a)
 {
-    __shared__ uint4 *s_dst[kRowBatch];
+    extern __shared__ int32_t sh[];
+    __shared__ int s_warp[kCountThreads / 32];
     pdl_trigger();
-    const int r = blockIdx.y, k = a.topk;
-    const int64_t t = blockIdx.x / a.nseg;
-    const int seg = (int)(blockIdx.x - t * a.nseg), per = (a.nvec + a.nseg - 1) / a.nseg, v1 = min(a.nvec, (seg + 1) * per);
-    const uint4 *src = (const uint4 *)a.x[r] + t * a.nvec;
+    const int E = a.n_experts, El = E / a.p, npairs = (int)a.tokens * a.topk, total = npairs * a.p;
+    int32_t *first = sh + a.p * E;
+    for (int i = threadIdx.x; i < a.p * E; i += kCountThreads) sh[i] = 0;
+    __syncthreads();
+    pdl_wait();
+    int ex[kRowsRegs], ps[kRowsRegs], rk[kRowsRegs];
+#pragma unroll
+    for (int k = 0; k < kRowsRegs; ++k) {
+        const int i = k * kCountThreads + threadIdx.x;
+        rk[k] = 0;
+        ex[k] = -1;
+        if (i < total) {
+            rk[k] = i / npairs;
+            ex[k] = a.idx[rk[k]][i - rk[k] * npairs];
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kRowsRegs; ++k) ps[k] = ex[k] >= 0 && ex[k] < E ? atomicAdd(&sh[rk[k] * E + ex[k]], 1) : -1;
+    __syncthreads();
+    int carry = 0;
+    for (int e0 = 0; e0 < E; e0 += kCountThreads) {  // first row of every expert, counting over all owners
+        const int e = e0 + threadIdx.x;
+        int t = 0;
+        if (e < E)
+            for (int r = 0; r < a.p; ++r) t += sh[r * E + e];
+        int all;
+        const int before = cta_prefix(t, s_warp, &all);
+        if (e < E) first[e] = carry + before;
+        carry += all;
+    }
+    if (threadIdx.x == 0) first[E] = carry;
+    __syncthreads();
+    for (int e = threadIdx.x; e < E; e += kCountThreads) {
+        const int q = e / El, f = first[q * El];
+        int row = first[e] - f;
+        a.expert_offsets[q][e - q * El] = row;
+        if (e == q * El + El - 1) {
+            const int rows = first[e + 1] - f;
+            a.expert_offsets[q][El] = rows;
+            *a.recv_rows[q] = rows;
+            if (rows > a.capacity) *a.overflow[q] = 1;
+        }
+        for (int r = 0; r < a.p; ++r) { const int c = sh[r * E + e]; sh[r * E + e] = row; row += c; }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kRowsRegs; ++k)
+        if (ps[k] >= 0) a.dst_row[rk[k]][k * kCountThreads + threadIdx.x - rk[k] * npairs] = sh[rk[k] * E + ex[k]] + ps[k];
+}
+
+// grid (tokens x segments, ranks); kRows: the rows are in dst_row already; V: vectors of 32 bytes where the rows allow them, else of 16
+template <class V, bool kRows>
+__global__ void __launch_bounds__(kDispatchThreads) moe_local_dispatch_kernel(const __grid_constant__ MoeTables a)
+{
+    constexpr int kPer = 128 / sizeof(V);  // 128 bytes of a row per thread and round
+    __shared__ V *s_dst[kRowBatch];
+    pdl_trigger();
+    const int r = blockIdx.y, k = a.topk, nvec = a.nvec / (int)(sizeof(V) / 16);
+    const int64_t t = a.nseg == 1 ? blockIdx.x : blockIdx.x / a.nseg;
+    const int seg = (int)(blockIdx.x - t * a.nseg), per = (nvec + a.nseg - 1) / a.nseg, v1 = min(nvec, (seg + 1) * per);
+    const V *src = (const V *)a.x[r] + t * nvec;
     pdl_wait();
     for (int k0 = 0; k0 < k; k0 += kRowBatch) {
         if (k0) __syncthreads();
+        V x[kPer];
+        const int v0 = seg * per + threadIdx.x;
+#pragma unroll
+        for (int u = 0; u < kPer; ++u)
+            if (v0 + u * kDispatchThreads < v1) x[u] = ld_row(src + v0 + u * kDispatchThreads);
         if (threadIdx.x < kRowBatch) {
-            uint4 *d = nullptr;
+            V *d = nullptr;
             if (k0 + (int)threadIdx.x < k) {
                 const int64_t i = t * k + k0 + threadIdx.x;
-                const int e = a.idx[r][i];
+                const int e = a.idx[r][i], known = kRows ? a.dst_row[r][i] : a.pos[r][i];
                 if (e >= 0 && e < a.n_experts) {
-                    const int64_t row = (int64_t)a.hist[((int64_t)r * a.nchunk + i / a.chunk) * a.n_experts + e] + a.pos[r][i];
-                    if (seg == 0) a.dst_row[r][i] = (int32_t)row;
-                    if (row < a.capacity) d = (uint4 *)a.rows[e / (a.n_experts / a.p)] + row * a.nvec;
+                    const int64_t row = kRows ? known : a.hist[((int64_t)r * a.nchunk + (uint32_t)i / (uint32_t)a.chunk) * a.n_experts + e] + known;
+                    if (!kRows && seg == 0) a.dst_row[r][i] = (int32_t)row;
+                    if (row < a.capacity) d = (V *)a.rows[e / (a.n_experts / a.p)] + row * nvec;
                 }
             }
             s_dst[threadIdx.x] = d;
         }
-        uint4 x[4];
-        const int v0 = seg * per + threadIdx.x;
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (v0 + u * kRowThreads < v1) x[u] = src[v0 + u * kRowThreads];
         __syncthreads();
         for (int vb = v0;;) {
 #pragma unroll
             for (int j = 0; j < kRowBatch; ++j) {
-                uint4 *d = s_dst[j];
+                V *d = s_dst[j];
                 if (!d) continue;
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (vb + u * kRowThreads < v1) d[vb + u * kRowThreads] = x[u];
+                for (int u = 0; u < kPer; ++u)
+                    if (vb + u * kDispatchThreads < v1) st_row(d + vb + u * kDispatchThreads, x[u]);
             }
-            vb += 4 * kRowThreads;
+            vb += kPer * kDispatchThreads;
             if (vb >= v1) break;
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (vb + u * kRowThreads < v1) x[u] = src[vb + u * kRowThreads];
+            for (int u = 0; u < kPer; ++u)
+                if (vb + u * kDispatchThreads < v1) x[u] = ld_row(src + vb + u * kDispatchThreads);
         }
     }
 }
@@ -218,10 +338,10 @@ __global__ void __launch_bounds__(kRowThreads) moe_local_combine_kernel(const __
 }
 
 // Parts of a row per CTA row: whole rows once there is a CTA for every SM several times over.
-int segments(int64_t units, int nvec)
+int segments(int64_t units, int nvec, int threads)
 {
     int s = 1;
-    while (s < 4 && units * s < 4 * 148 && nvec / (2 * s) >= kRowThreads) s *= 2;
+    while (s < 4 && units * s < 4 * 148 && nvec / (2 * s) >= threads) s *= 2;
     return s;
 }
 
@@ -231,7 +351,6 @@ void fill(MoeTables &t, const MoeLocalLayer &l)
     moe_local_chunks(l.tokens * l.topk, &t.chunk, &t.nchunk);
     t.hist = l.scratch + 4;
     t.arrived = (uint32_t *)l.scratch;
-    t.nseg = segments(l.tokens * l.p, t.nvec);
     for (int q = 0; q < l.p; ++q) { t.pos[q] = l.pos[q]; t.dst_row[q] = l.dst_row[q]; }
 }
 
@@ -253,10 +372,21 @@ HcclResult moe_local_dispatch(const MoeLocalLayer &l, void *const *recv, const v
         t.x[q] = (const __nv_bfloat16 *)x[q]; t.idx[q] = idx[q]; t.rows[q] = (__nv_bfloat16 *)recv[q];
         t.expert_offsets[q] = l.expert_offsets[q]; t.recv_rows[q] = l.recv_rows[q]; t.overflow[q] = l.overflow[q];
     }
-    HcclResult rc = launch_pdl((const void *)moe_local_count_kernel, dim3((unsigned)t.nchunk, (unsigned)l.p), kCountThreads,
-                               sizeof(int32_t) * (l.n_experts + 1), &t, stream, "moe count");
+    // one CTA for all ranks' pairs while a thread can keep its own in registers and the counters fit shared memory
+    const size_t rows_smem = sizeof(int32_t) * ((size_t)l.p * l.n_experts + l.n_experts + 1);
+    const bool rows = l.tokens * l.topk * l.p <= kRowsRegs * kCountThreads && rows_smem <= 48 * 1024 - 256;
+    HcclResult rc = rows ? launch_pdl((const void *)moe_local_rows_kernel, dim3(1), kCountThreads, rows_smem, &t, stream, "moe rows")
+                         : launch_pdl((const void *)moe_local_count_kernel, dim3((unsigned)t.nchunk, (unsigned)l.p), kCountThreads,
+                                      sizeof(int32_t) * (l.n_experts + 1 + std::max(1, kCountThreads / l.n_experts) * l.n_experts), &t, stream, "moe count");
     if (rc != HCCL_SUCCESS) return rc;
-    return launch_pdl((const void *)moe_local_dispatch_kernel, dim3((unsigned)(l.tokens * t.nseg), (unsigned)l.p), kRowThreads, 0, &t, stream, "moe dispatch");
+    uintptr_t bits = (uintptr_t)(l.hidden * 2);
+    for (int q = 0; q < l.p; ++q) bits |= (uintptr_t)x[q] | (uintptr_t)recv[q];
+    const bool wide = (bits & 31) == 0;
+    t.nseg = segments(l.tokens * l.p, wide ? t.nvec / 2 : t.nvec, kDispatchThreads);
+    const void *fn = wide ? (rows ? (const void *)moe_local_dispatch_kernel<Row32, true> : (const void *)moe_local_dispatch_kernel<Row32, false>)
+                          : (rows ? (const void *)moe_local_dispatch_kernel<uint4, true> : (const void *)moe_local_dispatch_kernel<uint4, false>);
+    return launch_pdl(fn,
+                      dim3((unsigned)(l.tokens * t.nseg), (unsigned)l.p), kDispatchThreads, 0, &t, stream, "moe dispatch");
 }
 
 HcclResult moe_local_combine(const MoeLocalLayer &l, void *const *rows, const int32_t *const *idx, const float *const *gates, void *const *out, void *stream)
@@ -266,6 +396,7 @@ HcclResult moe_local_combine(const MoeLocalLayer &l, void *const *rows, const in
     MoeTables t;
     fill(t, l);
     for (int q = 0; q < l.p; ++q) { t.idx[q] = idx[q]; t.rows[q] = (__nv_bfloat16 *)rows[q]; t.gates[q] = gates[q]; t.out[q] = (__nv_bfloat16 *)out[q]; }
+    t.nseg = segments(l.tokens * l.p, t.nvec, kRowThreads);
     return launch_pdl((const void *)moe_local_combine_kernel, dim3((unsigned)(l.tokens * t.nseg), (unsigned)l.p), kRowThreads, 0, &t, stream, "moe combine");
 }
 

@@ -80,7 +80,7 @@ extern HcclResult HcclB200MoeCombine(void *const *yPeers, const int32_t *topkIdx
 /* The same exchange for a communicator whose ranks are all in this process on one GPU (one rank included): counting, row bases
  * and dispatch of every rank in two launches, combine of every rank in one, ordered by the stream.  The tables hold one device
  * pointer per rank and stay the caller's; `scratch` has HcclB200MoeScratchBytes() bytes, zero before the first call, and
- * belongs to one exchange (one stream at a time).  HCCL_E_NOT_SUPPORT on other communicators or above 8192 experts. */
+ * belongs to one exchange (one stream at a time).  HCCL_E_NOT_SUPPORT on other communicators or above 4096 experts. */
 typedef struct HcclB200MoeLayerDef {
     int64_t tokens, capacityRows;       /* tokens of one rank, rows of one receive buffer */
     int32_t topk, hidden, nExperts, reserved;

@@ -54,7 +54,7 @@ class MoEExchange:
 
     def _local_layer(self, device):
         """Tables of the launches that serve all ranks at once, where all of them are in this process on one GPU."""
-        if not (self.comm.device and self.nl == self.p and self.E <= 8192):
+        if not (self.comm.device and self.nl == self.p and self.E <= 4096):
             return None
         self._scratch = torch.zeros(L.lib().HcclB200MoeScratchBytes(self.p, self.T, self.k, self.E) // 4, device=device, dtype=torch.int32)
         y = L.MoeLayer(tokens=self.T, capacityRows=self.cap, topk=self.k, hidden=self.H, nExperts=self.E, scratch=self._scratch.data_ptr())
