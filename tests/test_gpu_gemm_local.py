@@ -34,10 +34,15 @@ def check(c, ref):
     assert bad.numel() == 0, "tiles off: %s" % bad[:8].tolist()
 
 
-# one tile, of one k step; one tile split in two (shares of 8 and 9 steps) and in four, single CTAs and pairs; few tiles, split in
-# four, two and not; an odd number of row blocks; a last wave of a few tiles behind whole ones (pair, single); full waves exactly
+# one k step, then one row block split along K; few tiles, split and not; an odd number of row blocks; a last wave of a few tiles
+# behind whole ones (pair, single); full waves exactly
 SHAPES = [(128, 256, 64), (128, 256, 1088), (128, 256, 8192), (256, 256, 1088), (256, 256, 8192), (384, 768, 4096), (128, 8192, 3584), (128, 16384, 1024),
           (1024, 2048, 2112), (2560, 2048, 1024), (3200, 2048, 704), (2048, 2560, 64), (18944, 256, 256)]
+# tiles of other widths than 256 columns: uneven column halves and a last tile of 64 (144 columns), several waves (192, last tile
+# of 64; pair 224), a last tile of 176 of 208, single tiles of 128 and 80 columns split in four, pair tiles split in three and two,
+# a last pair tile of 32 columns of 224
+SHAPES += [(640, 4096, 2752), (640, 11008, 1024), (128, 28672, 1024), (384, 1280, 8192), (128, 2560, 8192), (256, 5120, 8192), (512, 3072, 4096),
+           (1280, 5632, 1024), (2048, 8192, 1024)]
 
 
 @pytest.mark.parametrize("M,N,K", SHAPES)
@@ -48,6 +53,20 @@ def test_product(M, N, K, act):
     c = fused_tp.gemm(a, b, activation=act)
     check(c, ref)
     assert torch.equal(fused_tp.gemm(a, b, activation=act), c)
+
+
+def test_silu_of_extreme_sums():
+    """Sums that are the values themselves: bf16 rounding of the result (2^-9) on top of a few fp32 steps; exponentials beyond 2^126."""
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    x = torch.tensor([0., -1e-30, 1e-30, -1., 1., -20., 20., -86., -87., -87.5, -88., -88.5, -89., -100., 100., 3e38, -3e38], device="cuda")
+    a = torch.zeros(128, 64, device="cuda", dtype=torch.bfloat16)
+    a[:x.numel(), 0] = x.to(torch.bfloat16)
+    b = torch.zeros(256, 64, device="cuda", dtype=torch.bfloat16)
+    b[:, 0] = 1
+    want = torch.nn.functional.silu(a[:, :1].float()).double().expand(128, 256)
+    got = fused_tp.gemm(a, b, activation="silu").double()
+    assert bool(((got - want).abs() <= want.abs() * 2 ** -8 + 2 ** -126).all()), got[:x.numel(), 0].tolist()
 
 
 def test_output_aligned_to_16_bytes_only():
