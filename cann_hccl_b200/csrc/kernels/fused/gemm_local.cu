@@ -4,8 +4,9 @@
 //   warp 1     one thread issues tcgen05.mma into one of two accumulators of up to 256 columns;
 //   warps 2-9  drain the other accumulator: two warps per TMEM lane quarter, half of the columns each, full 32-byte sectors per store.
 // Pair form: a cluster of two CTAs shares a tile of 256 rows (cta_group::2), each CTA loading its 128 rows of A and half of the
-// tile's B rows; single form: one CTA per 128 rows.  A tile has 64 to 256 columns: the width, the form and the split follow
-// from the shape (tiling_ns), so that the tiles fill whole waves of the GPU.
+// tile's B rows; single form: one CTA per 128 rows.  The two row blocks of a pair may belong to different ranks, and with an odd
+// number of them the last pair computes one block of zeros.  A tile has 64 to 256 columns: the width, the form and the split
+// follow from the shape (tiling_ns), so that the tiles fill whole waves of the GPU.
 //
 // Few tiles (a decode batch: one row block, deep K): a cluster of S units shares a tile along K (kSplit).  Each unit leaves
 // its fp32 sums in its shared memory, the cluster meets, and the units take groups of 16 columns in turn, adding the S copies
@@ -48,6 +49,7 @@ struct alignas(64) GemmParams {
     int form, act;
     int cols;                        // columns of a tile: multiple of 16, pair: of 32
     int um_tiles, n_tiles, shard_tiles;  // row units (128 rows, pair: 256), column tiles, column tiles of one shard (the last may be narrower)
+    int rows, shards;                // rows of the tile space (pair: the last unit may be half outside), shards of A (gather)
     int shard_m, shard_n;            // rows of a row shard, columns of a column shard
     int k_seg, k_iters;              // k steps of one operand pair, of a whole tile
     int ldc, panel;                  // panel: n tiles that are walked together
@@ -109,7 +111,7 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr)
     return v;
 }
 
-// address of (row, column of shard sn) in its rank's output
+// address of (row, column of shard sn) in its rank's output; row lies inside the tile space
 __device__ __forceinline__ __nv_bfloat16 *out_row(const GemmParams &P, int row, int sn, int col)
 {
     if (P.form == GEMM_GATHER) return P.C[sn] + (int64_t)row * P.ldc + col;
@@ -171,7 +173,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_local_kernel(const __gri
                 const int brow = w.col + (kPair ? (int)cta_r * (P.cols / 2) : 0);
                 const CUtensorMap *ma = &P.tmA[0], *mb = &P.tmB[0];
                 if (P.form == GEMM_GATHER) {
-                    const int sm = arow / P.shard_m;
+                    const int sm = min(arow / P.shard_m, P.shards - 1);  // past the last row: zeros
                     ma = &P.tmA[sm]; arow -= sm * P.shard_m;
                     mb = &P.tmB[w.sn];
                 }
@@ -226,8 +228,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_local_kernel(const __gri
         uint32_t n = 0;
         for (int t = unit; t < total && !*fail; t += P.units, ++n) {
             const Tile w = tile_at(P, t);
-            __nv_bfloat16 *dst = out_row(P, (w.um * kCtas + (int)cta_r) * BM + rl, w.sn, w.col);
-            const int c_end = min(c_hi, P.shard_n - w.col);  // a shard's last tile may be narrower
+            const int row0 = (w.um * kCtas + (int)cta_r) * BM;
+            const int c_end = row0 < P.rows ? min(c_hi, P.shard_n - w.col) : 0;  // a shard's last tile may be narrower
+            __nv_bfloat16 *dst = row0 < P.rows ? out_row(P, row0 + rl, w.sn, w.col) : nullptr;
             const uint32_t buf = n & 1, use = n >> 1, taddr = tmem_base + buf * kMaxCols + ((uint32_t)(q4 * 32) << 16);
             if (!mbar_wait_t<kPair>(&S.tmem_full[buf], use & 1, fail)) break;
             tc_fence_after();
@@ -278,8 +281,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_local_kernel(const __gri
         cluster_sync_all();
         if (warp >= 2) {  // groups of 16 columns in turn over the units and their column halves
             const Tile w = tile_at(P, unit);
-            __nv_bfloat16 *dst = out_row(P, (w.um * kCtas + (int)cta_r) * BM + rl, w.sn, w.col);
-            const int c_end = min(P.cols, P.shard_n - w.col);
+            const int row0 = (w.um * kCtas + (int)cta_r) * BM;
+            const int c_end = row0 < P.rows ? min(P.cols, P.shard_n - w.col) : 0;
+            __nv_bfloat16 *dst = row0 < P.rows ? out_row(P, row0 + rl, w.sn, w.col) : nullptr;
 #pragma unroll 1
             for (int c = 16 * (2 * share + half); c < c_end; c += 32 * split) {
                 const uint32_t own = smem_u32(sums + (c / 4) * BM + rl);
@@ -402,7 +406,7 @@ bool shape_ok(const GemmCall &c)
 }
 
 // Row units and column tiles of a call under a tiling.
-int row_units(const GemmCall &c, bool pair) { return c.M / (pair ? 2 * BM : BM); }
+int row_units(const GemmCall &c, bool pair) { return pair ? (c.M + 2 * BM - 1) / (2 * BM) : c.M / BM; }
 int shard_tiles(const GemmCall &c, int cols) { return (c.N + cols - 1) / cols; }
 
 // Estimated time (ns) of a tiling: the slowest unit (its rows of A and B per k step, which L2 delivers at 128 bytes per 0.8 to
@@ -485,7 +489,9 @@ HcclResult launch_gemm_local(const GemmCall &c, DevStatus *status, void *stream)
     DeviceShape d;
     CHK_RET(device_shape(&d));
     const int na = c.form == GEMM_PLAIN ? 1 : c.p, rows = c.form == GEMM_PLAIN ? c.M : c.M / c.p;
-    const Tiling til = tiling_for(c, d, env_config().tp_gemm_pair && rows % (2 * BM) == 0);
+    // an odd number of row blocks leaves a block of zeros in the last pair: worth it from eight row units on (7040 x 4352 x 5632
+    // 252 -> 234 us, 2176 x 20992 x 6400 425 -> 392), not below (1152 x 2560 x 4864 22.5 -> 23.9, 640 x 11008 x 4096 46.5 -> 56.4)
+    const Tiling til = tiling_for(c, d, env_config().tp_gemm_pair && (c.M / BM % 2 == 0 || c.M > 15 * BM));
     const bool pair = til.pair;
     GemmParams P;
     memset(&P, 0, sizeof(P));
@@ -510,6 +516,7 @@ HcclResult launch_gemm_local(const GemmCall &c, DevStatus *status, void *stream)
     P.wide = (bits & 31) == 0;
     P.status = status;
     P.form = c.form; P.act = c.act;
+    P.rows = c.M; P.shards = na;
     P.shard_m = rows;
     P.shard_n = c.N;
     P.ldc = c.N;

@@ -43,6 +43,8 @@ SHAPES = [(128, 256, 64), (128, 256, 1088), (128, 256, 8192), (256, 256, 1088), 
 # a last pair tile of 32 columns of 224
 SHAPES += [(640, 4096, 2752), (640, 11008, 1024), (128, 28672, 1024), (384, 1280, 8192), (128, 2560, 8192), (256, 5120, 8192), (512, 3072, 4096),
            (1280, 5632, 1024), (2048, 8192, 1024)]
+# pairs over an odd number of row blocks, the last half empty; just below the size from which they are used
+SHAPES += [(2176, 1024, 512), (2176, 8192, 192), (1920, 2048, 512)]
 
 
 @pytest.mark.parametrize("M,N,K", SHAPES)
@@ -79,7 +81,7 @@ def test_output_aligned_to_16_bytes_only():
 
 
 @pytest.mark.parametrize("p", [2, 3, 4])
-@pytest.mark.parametrize("Ms,N,K", [(128, 256, 64), (256, 1024, 1152), (384, 512, 2048)])
+@pytest.mark.parametrize("Ms,N,K", [(128, 256, 64), (256, 1024, 1152), (384, 512, 2048), (1152, 2048, 1024)])
 def test_layers_of_local_ranks(p, Ms, N, K):
     xs, ws = operands(Ms, N, K, p + N, p)
     cfg = L.CommConfig.default()
