@@ -7,12 +7,14 @@
 //             receive rows: tokens x (1 + k) rows of traffic, the least the exchange can do;
 //   combine   the same split over the output rows: eight expert rows in flight per thread, fp32 sum in k order, one rounding.
 //
-// A decode batch (8192 pairs and fewer over all ranks) has its rows from ONE CTA that counts in shared memory and registers.
+// Up to 65536 pairs over all ranks, the rows come from ONE cluster that counts in shared memory and registers; the dispatch
+// loads its activations and experts meanwhile.
 //
 // Bound: HBM for prefill batches (8192 tokens x 7168, top 8, one rank: dispatch 165 us at 6.4 TB/s, combine 156 us at 6.8 TB/s,
-// whole exchange 338 us, 468 us with a row read per expert, a launch per rank and step, and barriers), launches and L2 for
-// decode batches (128 tokens on each of four ranks: 26 us, 301 us before).  Dispatch with 16-byte instead of 32-byte vectors:
-// 171 us; counting a decode batch with the prefill kernel: 9 us instead of 5.6 us.
+// whole exchange 337 us, 468 us with a row read per expert, a launch per rank and step, and barriers), launches and L2 for
+// decode batches (128 tokens on each of four ranks: 25 us, 301 us before).  Dispatch with 16-byte instead of 32-byte vectors:
+// 171 us.  Rows of 7224 pairs: 1 CTA 16.3 us for the whole exchange (903 tokens x 1280), four CTAs 15.1 us; 65536 pairs counted
+// through global memory: 340 us, by the cluster 338 us.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <algorithm>
@@ -25,7 +27,7 @@ namespace hcclb {
 
 namespace {
 
-constexpr int kCountThreads = 1024, kScanRegs = 16, kRowsRegs = 8, kDispatchThreads = 128, kRowThreads = 256, kRowBatch = 8;
+constexpr int kCountThreads = 1024, kScanRegs = 16, kRowsRegs = 8, kRowsCluster = 8, kDispatchThreads = 128, kRowThreads = 256, kRowBatch = 8;
 
 struct alignas(32) Row32 { uint32_t w[8]; };
 __device__ __forceinline__ uint4 ld_row(const uint4 *p) { return *p; }
@@ -66,6 +68,17 @@ __device__ __forceinline__ int cta_prefix(int t, int *s_warp, int *all)
     return before + v - t;
 }
 
+// The totals that the cluster's CTAs leave for each other.
+__device__ __forceinline__ void moe_cluster_sync() { asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ int ld_cluster_s32(const int32_t *own, int cta)
+{
+    uint32_t at;
+    int v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(own)), "r"(cta));
+    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
+    return v;
+}
+
 struct MoeTables {
     const __nv_bfloat16 *x[kMaxRanks];
     const int32_t *idx[kMaxRanks];
@@ -84,12 +97,12 @@ __global__ void __launch_bounds__(kCountThreads) moe_local_count_kernel(const __
 {
     extern __shared__ int32_t sh[];  // [experts + 1], then [parts][experts]
     __shared__ int s_last;
-    pdl_trigger();
     const int E = a.n_experts, r = blockIdx.y;
     const int64_t npairs = a.tokens * a.topk, i0 = (int64_t)blockIdx.x * a.chunk, i1 = min(i0 + a.chunk, npairs);
     for (int e = threadIdx.x; e < E; e += kCountThreads) sh[e] = 0;
     __syncthreads();
     pdl_wait();
+    pdl_trigger();  // from here on the dispatch may read what this kernel found complete: activations and experts
     for (int64_t i = i0 + threadIdx.x; i < i1; i += kCountThreads) {
         const int e = a.idx[r][i];
         a.pos[r][i] = e >= 0 && e < E ? atomicAdd(&sh[e], 1) : -1;
@@ -163,26 +176,28 @@ __global__ void __launch_bounds__(kCountThreads) moe_local_count_kernel(const __
     }
 }
 
-// Few pairs (a decode batch): one CTA numbers the pairs of all ranks and knows their rows without a trip through global memory
-// (no histogram, no fence, no arrival).  A thread keeps its pairs in registers.  Dynamic shared memory: [rank][expert] counters,
-// then their first rows; [experts + 1] first row of an expert over all owners.
+// Up to 65536 pairs: one cluster numbers the pairs of all ranks and knows their rows without a trip through global memory (no
+// histogram, no fence, no arrival).  CTA c takes a stretch of the pairs in rank order, a thread keeps its pairs in registers,
+// and the CTAs read each other's totals per expert through distributed shared memory.  Dynamic shared memory: [rank][expert]
+// counters, then first rows; [experts + 1] first row of an expert over all owners; [experts] pairs of this CTA.
 __global__ void __launch_bounds__(kCountThreads) moe_local_rows_kernel(const __grid_constant__ MoeTables a)
 {
     extern __shared__ int32_t sh[];
     __shared__ int s_warp[kCountThreads / 32];
-    pdl_trigger();
     const int E = a.n_experts, El = E / a.p, npairs = (int)a.tokens * a.topk, total = npairs * a.p;
-    int32_t *first = sh + a.p * E;
+    const int ctas = (int)gridDim.x, c = (int)blockIdx.x, per = (total + ctas - 1) / ctas, i0 = c * per, i1 = min(total, i0 + per);
+    int32_t *first = sh + a.p * E, *mine = first + E + 1;
     for (int i = threadIdx.x; i < a.p * E; i += kCountThreads) sh[i] = 0;
     __syncthreads();
     pdl_wait();
+    pdl_trigger();  // from here on the dispatch may read what this kernel found complete: activations and experts
     int ex[kRowsRegs], ps[kRowsRegs], rk[kRowsRegs];
 #pragma unroll
     for (int k = 0; k < kRowsRegs; ++k) {
-        const int i = k * kCountThreads + threadIdx.x;
+        const int i = i0 + k * kCountThreads + (int)threadIdx.x;
         rk[k] = 0;
         ex[k] = -1;
-        if (i < total) {
+        if (i < i1) {
             rk[k] = i / npairs;
             ex[k] = a.idx[rk[k]][i - rk[k] * npairs];
         }
@@ -190,35 +205,57 @@ __global__ void __launch_bounds__(kCountThreads) moe_local_rows_kernel(const __g
 #pragma unroll
     for (int k = 0; k < kRowsRegs; ++k) ps[k] = ex[k] >= 0 && ex[k] < E ? atomicAdd(&sh[rk[k] * E + ex[k]], 1) : -1;
     __syncthreads();
+    if (ctas > 1) {
+        for (int e = threadIdx.x; e < E; e += kCountThreads) {
+            int t = 0;
+            for (int r = 0; r < a.p; ++r) t += sh[r * E + e];
+            mine[e] = t;
+        }
+        moe_cluster_sync();
+    }
     int carry = 0;
     for (int e0 = 0; e0 < E; e0 += kCountThreads) {  // first row of every expert, counting over all owners
         const int e = e0 + threadIdx.x;
-        int t = 0;
-        if (e < E)
-            for (int r = 0; r < a.p; ++r) t += sh[r * E + e];
+        int t = 0, earlier = 0;  // pairs of the expert, of them those of earlier CTAs
+        if (e < E) {
+            if (ctas > 1) {
+                int n[kRowsCluster];
+#pragma unroll
+                for (int q = 0; q < kRowsCluster; ++q) n[q] = q < ctas ? ld_cluster_s32(mine + e, q) : 0;
+#pragma unroll
+                for (int q = 0; q < kRowsCluster; ++q) { t += n[q]; earlier += q < c ? n[q] : 0; }
+            } else
+                for (int r = 0; r < a.p; ++r) t += sh[r * E + e];
+        }
         int all;
         const int before = cta_prefix(t, s_warp, &all);
-        if (e < E) first[e] = carry + before;
+        if (e < E) {
+            first[e] = carry + before;
+            int row = earlier;  // counted from the expert's first row
+            for (int r = 0; r < a.p; ++r) { const int k = sh[r * E + e]; sh[r * E + e] = row; row += k; }
+        }
         carry += all;
     }
     if (threadIdx.x == 0) first[E] = carry;
     __syncthreads();
-    for (int e = threadIdx.x; e < E; e += kCountThreads) {
-        const int q = e / El, f = first[q * El];
-        int row = first[e] - f;
-        a.expert_offsets[q][e - q * El] = row;
-        if (e == q * El + El - 1) {
-            const int rows = first[e + 1] - f;
-            a.expert_offsets[q][El] = rows;
-            *a.recv_rows[q] = rows;
-            if (rows > a.capacity) *a.overflow[q] = 1;
+    if (c == 0)
+        for (int e = threadIdx.x; e < E; e += kCountThreads) {
+            const int q = e / El, f = first[q * El];
+            a.expert_offsets[q][e - q * El] = first[e] - f;
+            if (e == q * El + El - 1) {
+                const int rows = first[e + 1] - f;
+                a.expert_offsets[q][El] = rows;
+                *a.recv_rows[q] = rows;
+                if (rows > a.capacity) *a.overflow[q] = 1;
+            }
         }
-        for (int r = 0; r < a.p; ++r) { const int c = sh[r * E + e]; sh[r * E + e] = row; row += c; }
-    }
-    __syncthreads();
 #pragma unroll
     for (int k = 0; k < kRowsRegs; ++k)
-        if (ps[k] >= 0) a.dst_row[rk[k]][k * kCountThreads + threadIdx.x - rk[k] * npairs] = sh[rk[k] * E + ex[k]] + ps[k];
+        if (ps[k] >= 0) {
+            const int e = ex[k];
+            a.dst_row[rk[k]][i0 + k * kCountThreads + (int)threadIdx.x - rk[k] * npairs] = first[e] - first[e / El * El] + sh[rk[k] * E + e] + ps[k];
+        }
+    if (ctas > 1) moe_cluster_sync();  // the others may still read this CTA's totals
 }
 
 // grid (tokens x segments, ranks); kRows: the rows are in dst_row already; V: vectors of 32 bytes where the rows allow them, else of 16
@@ -228,23 +265,32 @@ __global__ void __launch_bounds__(kDispatchThreads) moe_local_dispatch_kernel(co
     constexpr int kPer = 128 / sizeof(V);  // 128 bytes of a row per thread and round
     __shared__ V *s_dst[kRowBatch];
     pdl_trigger();
-    const int r = blockIdx.y, k = a.topk, nvec = a.nvec / (int)(sizeof(V) / 16);
+    const int r = blockIdx.y, k = a.topk, nvec = a.nvec / (int)(sizeof(V) / 16), nt = (int)blockDim.x;
     const int64_t t = a.nseg == 1 ? blockIdx.x : blockIdx.x / a.nseg;
     const int seg = (int)(blockIdx.x - t * a.nseg), per = (nvec + a.nseg - 1) / a.nseg, v1 = min(nvec, (seg + 1) * per);
     const V *src = (const V *)a.x[r] + t * nvec;
+    // the kernel before this one (rows or count) lets it start only after its own wait, and writes neither activations nor
+    // experts: they are loaded while it works
+    const int v0 = seg * per + threadIdx.x;
+    V x[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; ++u)
+        if (v0 + u * nt < v1) x[u] = ld_row(src + v0 + u * nt);
+    int e0 = -1;
+    if (threadIdx.x < kRowBatch && (int)threadIdx.x < k) e0 = a.idx[r][t * k + threadIdx.x];
     pdl_wait();
     for (int k0 = 0; k0 < k; k0 += kRowBatch) {
-        if (k0) __syncthreads();
-        V x[kPer];
-        const int v0 = seg * per + threadIdx.x;
+        if (k0) {
+            __syncthreads();
 #pragma unroll
-        for (int u = 0; u < kPer; ++u)
-            if (v0 + u * kDispatchThreads < v1) x[u] = ld_row(src + v0 + u * kDispatchThreads);
+            for (int u = 0; u < kPer; ++u)
+                if (v0 + u * nt < v1) x[u] = ld_row(src + v0 + u * nt);
+        }
         if (threadIdx.x < kRowBatch) {
             V *d = nullptr;
             if (k0 + (int)threadIdx.x < k) {
                 const int64_t i = t * k + k0 + threadIdx.x;
-                const int e = a.idx[r][i], known = kRows ? a.dst_row[r][i] : a.pos[r][i];
+                const int known = kRows ? a.dst_row[r][i] : a.pos[r][i], e = k0 ? a.idx[r][i] : e0;
                 if (e >= 0 && e < a.n_experts) {
                     const int64_t row = kRows ? known : a.hist[((int64_t)r * a.nchunk + (uint32_t)i / (uint32_t)a.chunk) * a.n_experts + e] + known;
                     if (!kRows && seg == 0) a.dst_row[r][i] = (int32_t)row;
@@ -261,13 +307,13 @@ __global__ void __launch_bounds__(kDispatchThreads) moe_local_dispatch_kernel(co
                 if (!d) continue;
 #pragma unroll
                 for (int u = 0; u < kPer; ++u)
-                    if (vb + u * kDispatchThreads < v1) st_row(d + vb + u * kDispatchThreads, x[u]);
+                    if (vb + u * nt < v1) st_row(d + vb + u * nt, x[u]);
             }
-            vb += kPer * kDispatchThreads;
+            vb += kPer * nt;
             if (vb >= v1) break;
 #pragma unroll
             for (int u = 0; u < kPer; ++u)
-                if (vb + u * kDispatchThreads < v1) x[u] = ld_row(src + vb + u * kDispatchThreads);
+                if (vb + u * nt < v1) x[u] = ld_row(src + vb + u * nt);
         }
     }
 }
@@ -303,7 +349,7 @@ __global__ void __launch_bounds__(kRowThreads) moe_local_combine_kernel(const __
         __syncthreads();
     };
     if (one) batch(0);
-    for (int vb = seg * per; vb < v1; vb += kRowThreads) {  // uniform trip count: the batches synchronise
+    for (int vb = seg * per; vb < v1; vb += blockDim.x) {  // uniform trip count: the batches synchronise
         const int v = vb + threadIdx.x;
         float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         for (int k0 = 0; k0 < k; k0 += kRowBatch) {
@@ -345,6 +391,14 @@ int segments(int64_t units, int nvec, int threads)
     return s;
 }
 
+// Threads of a CTA that goes through n vectors in the same number of rounds as `most` threads would, none of them half empty
+// (a row of 2816 bf16, 352 vectors: two rounds of 192 threads instead of 256 and 96).
+unsigned row_threads(int n, int most)
+{
+    const int rounds = std::max(1, (n + most - 1) / most);
+    return (unsigned)std::max(32, ((n + rounds - 1) / rounds + 31) / 32 * 32);
+}
+
 void fill(MoeTables &t, const MoeLocalLayer &l)
 {
     t.p = l.p; t.topk = l.topk; t.nvec = l.hidden / 8; t.n_experts = l.n_experts; t.tokens = l.tokens; t.capacity = l.capacity;
@@ -372,10 +426,13 @@ HcclResult moe_local_dispatch(const MoeLocalLayer &l, void *const *recv, const v
         t.x[q] = (const __nv_bfloat16 *)x[q]; t.idx[q] = idx[q]; t.rows[q] = (__nv_bfloat16 *)recv[q];
         t.expert_offsets[q] = l.expert_offsets[q]; t.recv_rows[q] = l.recv_rows[q]; t.overflow[q] = l.overflow[q];
     }
-    // one CTA for all ranks' pairs while a thread can keep its own in registers and the counters fit shared memory
-    const size_t rows_smem = sizeof(int32_t) * ((size_t)l.p * l.n_experts + l.n_experts + 1);
-    const bool rows = l.tokens * l.topk * l.p <= kRowsRegs * kCountThreads && rows_smem <= 48 * 1024 - 256;
-    HcclResult rc = rows ? launch_pdl((const void *)moe_local_rows_kernel, dim3(1), kCountThreads, rows_smem, &t, stream, "moe rows")
+    // one cluster for all ranks' pairs while a thread can keep its own in registers and the counters fit shared memory: a CTA
+    // for every 2048 pairs (up to eight), one alone up to 4096, where meeting the others costs what it saves
+    const size_t rows_smem = sizeof(int32_t) * ((size_t)l.p * l.n_experts + 2 * l.n_experts + 1);
+    const int64_t total = l.tokens * l.topk * l.p;
+    const bool rows = total <= kRowsCluster * kRowsRegs * kCountThreads && rows_smem <= 48 * 1024 - 256;
+    const int ctas = rows && total > 4096 ? (int)std::min<int64_t>(kRowsCluster, (total + 2047) / 2048) : 1;
+    HcclResult rc = rows ? launch_pdl((const void *)moe_local_rows_kernel, dim3((unsigned)ctas), kCountThreads, rows_smem, &t, stream, "moe rows", ctas)
                          : launch_pdl((const void *)moe_local_count_kernel, dim3((unsigned)t.nchunk, (unsigned)l.p), kCountThreads,
                                       sizeof(int32_t) * (l.n_experts + 1 + std::max(1, kCountThreads / l.n_experts) * l.n_experts), &t, stream, "moe count");
     if (rc != HCCL_SUCCESS) return rc;
@@ -385,8 +442,8 @@ HcclResult moe_local_dispatch(const MoeLocalLayer &l, void *const *recv, const v
     t.nseg = segments(l.tokens * l.p, wide ? t.nvec / 2 : t.nvec, kDispatchThreads);
     const void *fn = wide ? (rows ? (const void *)moe_local_dispatch_kernel<Row32, true> : (const void *)moe_local_dispatch_kernel<Row32, false>)
                           : (rows ? (const void *)moe_local_dispatch_kernel<uint4, true> : (const void *)moe_local_dispatch_kernel<uint4, false>);
-    return launch_pdl(fn,
-                      dim3((unsigned)(l.tokens * t.nseg), (unsigned)l.p), kDispatchThreads, 0, &t, stream, "moe dispatch");
+    const int nv = wide ? t.nvec / 2 : t.nvec;
+    return launch_pdl(fn, dim3((unsigned)(l.tokens * t.nseg), (unsigned)l.p), row_threads((nv + t.nseg - 1) / t.nseg, kDispatchThreads), 0, &t, stream, "moe dispatch");
 }
 
 HcclResult moe_local_combine(const MoeLocalLayer &l, void *const *rows, const int32_t *const *idx, const float *const *gates, void *const *out, void *stream)
@@ -397,7 +454,8 @@ HcclResult moe_local_combine(const MoeLocalLayer &l, void *const *rows, const in
     fill(t, l);
     for (int q = 0; q < l.p; ++q) { t.idx[q] = idx[q]; t.rows[q] = (__nv_bfloat16 *)rows[q]; t.gates[q] = gates[q]; t.out[q] = (__nv_bfloat16 *)out[q]; }
     t.nseg = segments(l.tokens * l.p, t.nvec, kRowThreads);
-    return launch_pdl((const void *)moe_local_combine_kernel, dim3((unsigned)(l.tokens * t.nseg), (unsigned)l.p), kRowThreads, 0, &t, stream, "moe combine");
+    return launch_pdl((const void *)moe_local_combine_kernel, dim3((unsigned)(l.tokens * t.nseg), (unsigned)l.p),
+                      row_threads((t.nvec + t.nseg - 1) / t.nseg, kRowThreads), 0, &t, stream, "moe combine");
 }
 
 }  // namespace hcclb
