@@ -5,7 +5,8 @@
 //             that finishes last turns all histograms into row bases, so nothing waits and no counter needs clearing first;
 //   dispatch  a CTA takes one token's row (or a part of it when tokens are few), reads it ONCE and stores it to its top-k
 //             receive rows: tokens x (1 + k) rows of traffic, the least the exchange can do;
-//   combine   the same split over the output rows: eight expert rows in flight per thread, fp32 sum in k order, one rounding.
+//   combine   the same split over the output rows, several tokens per CTA where top-k is small: eight expert rows in flight
+//             per thread, fp32 sum in k order, one rounding.
 //
 // Up to 65536 pairs over all ranks, the rows come from ONE cluster that counts in shared memory and registers; the dispatch
 // loads its activations and experts meanwhile.
@@ -14,7 +15,8 @@
 // whole exchange 337 us, 468 us with a row read per expert, a launch per rank and step, and barriers), launches and L2 for
 // decode batches (128 tokens on each of four ranks: 25 us, 301 us before).  Dispatch with 16-byte instead of 32-byte vectors:
 // 171 us.  Rows of 7224 pairs: 1 CTA 16.3 us for the whole exchange (903 tokens x 1280), four CTAs 15.1 us; 65536 pairs counted
-// through global memory: 340 us, by the cluster 338 us.
+// through global memory: 340 us, by the cluster 338 us.  Combine of 6516 tokens x 3840, top 4, with one token per CTA: 51 us, with
+// two 45 us; 32-byte instead of 16-byte loads cost occupancy (8192 x 7168, top 8: 159 -> 171 us).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <algorithm>
@@ -318,29 +320,35 @@ __global__ void __launch_bounds__(kDispatchThreads) moe_local_dispatch_kernel(co
     }
 }
 
-// grid (tokens x segments, ranks)
+// grid (groups of G tokens x segments, ranks).  A thread has eight expert rows in flight: B = 8 / G of each token of the group, so
+// that a small top-k does not leave it with two or four (the addresses of a group's rows are one round trip as well).
+template <int G>
 __global__ void __launch_bounds__(kRowThreads) moe_local_combine_kernel(const __grid_constant__ MoeTables a)
 {
+    constexpr int B = kRowBatch / G;
     __shared__ const uint4 *s_src[kRowBatch];
     __shared__ float s_gate[kRowBatch];
     pdl_trigger();
-    const int r = blockIdx.y, k = a.topk;
-    const int64_t t = blockIdx.x / a.nseg;
-    const int seg = (int)(blockIdx.x - t * a.nseg), per = (a.nvec + a.nseg - 1) / a.nseg, v1 = min(a.nvec, (seg + 1) * per);
-    uint4 *out = (uint4 *)a.out[r] + t * a.nvec;
+    const int r = blockIdx.y, k = a.topk, nt = (int)blockDim.x;
+    const int64_t t0 = (int64_t)(blockIdx.x / a.nseg) * G;
+    const int seg = (int)(blockIdx.x % a.nseg), per = (a.nvec + a.nseg - 1) / a.nseg, v1 = min(a.nvec, (seg + 1) * per);
+    uint4 *out = (uint4 *)a.out[r] + t0 * a.nvec;
     pdl_wait();
-    const bool one = k <= kRowBatch;
+    const bool one = k <= B;
     auto batch = [&](int k0) {
         if (threadIdx.x < kRowBatch) {
             const uint4 *s = nullptr;
             float g = 0.f;
-            if (k0 + (int)threadIdx.x < k) {
-                const int64_t i = t * k + k0 + threadIdx.x;
+            const int64_t t = t0 + threadIdx.x / B;
+            const int kk = k0 + threadIdx.x % B;
+            if (kk < k && t < a.tokens) {
+                const int64_t i = t * k + kk;
                 const int e = a.idx[r][i];
                 const int64_t row = a.dst_row[r][i];
+                const float gate = a.gates[r][i];
                 if (e >= 0 && e < a.n_experts && row >= 0 && row < a.capacity) {
                     s = (const uint4 *)a.rows[e / (a.n_experts / a.p)] + row * a.nvec;
-                    g = a.gates[r][i];
+                    g = gate;
                 }
             }
             s_src[threadIdx.x] = s;
@@ -349,10 +357,14 @@ __global__ void __launch_bounds__(kRowThreads) moe_local_combine_kernel(const __
         __syncthreads();
     };
     if (one) batch(0);
-    for (int vb = seg * per; vb < v1; vb += blockDim.x) {  // uniform trip count: the batches synchronise
-        const int v = vb + threadIdx.x;
-        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        for (int k0 = 0; k0 < k; k0 += kRowBatch) {
+    for (int vb = seg * per; vb < v1; vb += nt) {  // uniform trip count: the batches synchronise
+        const int v = vb + (int)threadIdx.x;
+        float acc[G][8];
+#pragma unroll
+        for (int u = 0; u < G; ++u)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[u][i] = 0.f;
+        for (int k0 = 0; k0 < k; k0 += B) {
             if (!one) { __syncthreads(); batch(k0); }
             if (v < v1) {
                 uint4 x[kRowBatch];
@@ -367,19 +379,21 @@ __global__ void __launch_bounds__(kRowThreads) moe_local_combine_kernel(const __
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const float2 f = __bfloat1622float2(h[i]);
-                        acc[2 * i] += g * f.x;
-                        acc[2 * i + 1] += g * f.y;
+                        acc[j / B][2 * i] += g * f.x;
+                        acc[j / B][2 * i + 1] += g * f.y;
                     }
                 }
             }
         }
-        if (v < v1) {
-            uint4 o;
-            __nv_bfloat162 *h = (__nv_bfloat162 *)&o;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(acc[2 * i], acc[2 * i + 1]);
-            out[v] = o;
-        }
+        for (int u = 0; u < G; ++u)
+            if (v < v1 && t0 + u < a.tokens) {
+                uint4 o;
+                __nv_bfloat162 *h = (__nv_bfloat162 *)&o;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(acc[u][2 * i], acc[u][2 * i + 1]);
+                out[(int64_t)u * a.nvec + v] = o;
+            }
     }
 }
 
@@ -453,9 +467,13 @@ HcclResult moe_local_combine(const MoeLocalLayer &l, void *const *rows, const in
     MoeTables t;
     fill(t, l);
     for (int q = 0; q < l.p; ++q) { t.idx[q] = idx[q]; t.rows[q] = (__nv_bfloat16 *)rows[q]; t.gates[q] = gates[q]; t.out[q] = (__nv_bfloat16 *)out[q]; }
-    t.nseg = segments(l.tokens * l.p, t.nvec, kRowThreads);
-    return launch_pdl((const void *)moe_local_combine_kernel, dim3((unsigned)(l.tokens * t.nseg), (unsigned)l.p),
-                      row_threads((t.nvec + t.nseg - 1) / t.nseg, kRowThreads), 0, &t, stream, "moe combine");
+    // tokens of a CTA: as many as eight rows in flight serve, while every SM keeps several CTAs
+    int group = kRowBatch / 2;
+    while (group > 1 && (group * l.topk > kRowBatch || l.tokens / group * l.p < 4 * 148)) group /= 2;
+    const int64_t groups = (l.tokens + group - 1) / group;
+    const void *fn = group == 4 ? (const void *)moe_local_combine_kernel<4> : group == 2 ? (const void *)moe_local_combine_kernel<2> : (const void *)moe_local_combine_kernel<1>;
+    t.nseg = segments(groups * l.p, t.nvec, kRowThreads);
+    return launch_pdl(fn, dim3((unsigned)(groups * t.nseg), (unsigned)l.p), row_threads((t.nvec + t.nseg - 1) / t.nseg, kRowThreads), 0, &t, stream, "moe combine");
 }
 
 }  // namespace hcclb

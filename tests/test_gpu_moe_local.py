@@ -11,10 +11,11 @@ pytestmark = pytest.mark.gpu
 
 
 # tokens x top-k around the chunk of 1024 pairs and beyond 32 chunks; top-k around the batch of eight rows; rows shorter than a
-# CTA, and longer than its four vectors per thread.  One CTA, clusters of two to eight, and more pairs or counters than they take
+# CTA, and longer than its four vectors per thread.  One CTA, clusters of two to eight, and more pairs or counters than they take.  CTAs of the
+# combine that take four and two tokens, the last one fewer
 @pytest.mark.parametrize("p,T,hidden,E,k", [(1, 1, 8, 4, 1), (1, 127, 264, 16, 8), (2, 129, 256, 64, 8), (3, 257, 2048, 33, 9), (4, 100, 8456, 8, 2),
                                             (1, 4100, 64, 256, 8), (8, 40, 512, 128, 17), (2, 33, 9216, 8, 2), (1, 1025, 16, 256, 8), (2, 512, 16, 1500, 8),
-                                            (4, 700, 32, 1024, 8), (8, 1024, 16, 32, 8), (1, 8300, 16, 64, 8), (3, 911, 2816, 48, 3), (8, 20, 16, 2048, 4)])
+                                            (4, 700, 32, 1024, 8), (8, 1024, 16, 32, 8), (1, 8300, 16, 64, 8), (3, 911, 2816, 48, 3), (8, 20, 16, 2048, 4), (1, 2371, 2816, 16, 2), (2, 593, 40, 16, 4)])
 @pytest.mark.parametrize("per_rank", [False, True])
 def test_exchange(p, T, hidden, E, k, per_rank):
     if not torch.cuda.is_available():
