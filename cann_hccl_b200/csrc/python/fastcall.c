@@ -54,6 +54,15 @@ static int addresses(PyObject *x, Py_ssize_t nlocal, void **out)
     return 0;
 }
 
+/* the same where every rank has a buffer: None is refused */
+static int all_addresses(PyObject *x, Py_ssize_t nlocal, void **out)
+{
+    if (addresses(x, nlocal, out)) return -1;
+    for (Py_ssize_t i = 0; i < nlocal; ++i)
+        if (!out[i]) { PyErr_SetString(PyExc_TypeError, "every rank needs a buffer, got None or one without memory"); return -1; }
+    return 0;
+}
+
 /* the caller has made these contiguous arrays of 64-bit unsigned integers */
 static int words(PyObject *x, Py_buffer *view, const uint64_t **out)
 {
@@ -200,7 +209,7 @@ static PyObject *moe_dispatch(PyObject *self, PyObject *const *a, Py_ssize_t n)
     if (PyErr_Occurred()) return NULL;
     if (nlocal < 1 || nlocal > MAX_LOCAL) { PyErr_SetString(PyExc_ValueError, "bad number of local ranks"); return NULL; }
     void *x[MAX_LOCAL], *idx[MAX_LOCAL];
-    if (addresses(a[3], nlocal, x) || addresses(a[4], nlocal, idx)) return NULL;
+    if (all_addresses(a[3], nlocal, x) || all_addresses(a[4], nlocal, idx)) return NULL;
     HcclResult rc;
     Py_BEGIN_ALLOW_THREADS
     rc = g_dispatch((HcclComm)comm, (const HcclB200MoeLayer *)layer, x, idx, (aclrtStream)stream);
@@ -217,7 +226,7 @@ static PyObject *moe_combine(PyObject *self, PyObject *const *a, Py_ssize_t n)
     if (PyErr_Occurred()) return NULL;
     if (nlocal < 1 || nlocal > MAX_LOCAL) { PyErr_SetString(PyExc_ValueError, "bad number of local ranks"); return NULL; }
     void *idx[MAX_LOCAL], *gates[MAX_LOCAL], *out[MAX_LOCAL];
-    if (addresses(a[4], nlocal, idx) || addresses(a[5], nlocal, gates) || addresses(a[6], nlocal, out)) return NULL;
+    if (all_addresses(a[4], nlocal, idx) || all_addresses(a[5], nlocal, gates) || all_addresses(a[6], nlocal, out)) return NULL;
     HcclResult rc;
     Py_BEGIN_ALLOW_THREADS
     rc = g_combine((HcclComm)comm, (const HcclB200MoeLayer *)layer, (void *const *)rows, idx, gates, out, (aclrtStream)stream);

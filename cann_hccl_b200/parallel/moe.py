@@ -104,6 +104,8 @@ class MoEExchange:
 
     def combine(self, gates, variant="mesh", source="expert_out", out=None):
         """gates: fp32 [tokens, topk].  source: 'expert_out' (after the experts ran) or 'recv' (identity experts)."""
+        if self._topk is None:
+            raise RuntimeError("combine() needs the routing of a dispatch()")
         gs = self._l(gates)
         if self._layer is not None:
             outs = self._l(out) if out is not None else [torch.empty(self.T, self.H, device=g.device, dtype=torch.bfloat16) for g in gs]

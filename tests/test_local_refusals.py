@@ -1,0 +1,73 @@
+"""Calls that the paths for ranks of one process have to refuse on the host, before anything is launched."""
+import ctypes as C
+
+import pytest
+
+import cann_hccl_b200 as H
+from cann_hccl_b200 import _lib as L
+
+PER_RANK = ("rows", "pos", "dstRow", "expertOffsets", "recvRows", "overflow")
+
+
+@pytest.fixture(scope="module")
+def pair():
+    c = H.Communicator.init_local(2, device=False)
+    yield c
+    c.destroy()
+
+
+def moe_call(comm, missing=None, rank=1, entry="dispatch"):
+    """A dispatch or combine of the host communicator's ranks, with one entry of one table null: result code.  Complete tables
+    come as far as the check of the transport (the launches need a GPU)."""
+    mem = C.create_string_buffer(64)
+    at = (C.addressof(mem) + 31) // 32 * 32
+    y = L.MoeLayer(tokens=4, capacityRows=8, topk=2, hidden=8, nExperts=4, scratch=at)
+    call = {n: (C.c_void_p * 2)(at, at) for n in ("x", "idx", "gates", "out", "given")}
+    for n in PER_RANK:
+        for r in range(2):
+            getattr(y, n)[r] = at
+    if missing == "scratch":
+        y.scratch = None
+    elif missing in PER_RANK:
+        getattr(y, missing)[rank] = None
+    elif missing:
+        call[missing][rank] = None
+    if entry == "dispatch":
+        return L.lib().HcclB200MoeDispatchLocal(comm.handle, C.byref(y), call["x"], call["idx"], None)
+    rows = call["given"] if missing == "given" else None
+    return L.lib().HcclB200MoeCombineLocal(comm.handle, C.byref(y), rows, call["idx"], call["gates"], call["out"], None)
+
+
+def test_moe_tables_with_a_null_entry(pair):
+    for entry, tables in (("dispatch", ("x", "idx")), ("combine", ("idx", "gates", "out", "given"))):
+        assert moe_call(pair, entry=entry) == L.E_NOT_SUPPORT
+        for name in PER_RANK + ("scratch",) + tables:
+            for rank in range(2):
+                assert moe_call(pair, name, rank, entry) == L.E_PTR, (entry, name, rank)
+
+
+@pytest.mark.parametrize("nlocal,bad", [(1, None), (1, [None]), (2, [None, None])])
+def test_moe_call_path_refuses_none(nlocal, bad):
+    """The Python call path, for a lone rank (which passes its buffer without a list) and for several: no communicator is reached."""
+    import numpy as np
+    good = [np.zeros(8, np.float32) for _ in range(nlocal)]
+    L.lib()
+    with pytest.raises(TypeError):
+        L.fast.moe_dispatch(0, nlocal, 0, bad, good, 0)
+    with pytest.raises(TypeError):
+        L.fast.moe_dispatch(0, nlocal, 0, good, bad, 0)
+    for at in range(3):
+        args = [good, good, good]
+        args[at] = bad
+        with pytest.raises(TypeError):
+            L.fast.moe_combine(0, nlocal, 0, 0, *args, 0)
+    assert L.fast.moe_combine(0, nlocal, 0, 0, good, good, good, 0) == L.E_PTR  # all buffers there: refused for the communicator
+
+
+def test_combine_before_any_dispatch():
+    pytest.importorskip("torch")
+    from cann_hccl_b200.parallel import moe
+    ex = object.__new__(moe.MoEExchange)
+    ex._topk = None
+    with pytest.raises(RuntimeError):
+        ex.combine(None)
