@@ -713,19 +713,25 @@ int64_t HcclB200MoeScratchBytes(int32_t nRanks, int64_t tokens, int32_t topk, in
 {
     return nRanks < 1 || tokens < 0 || topk < 1 || nExperts < 1 ? -1 : moe_local_scratch_words(nRanks, tokens, topk, nExperts) * 4;
 }
-// The tables of a layer and of a call (x and topkIdx; rows, topkIdx, gates and out): an entry for every rank, none of them null.
-static HcclResult moe_layer(Communicator *c, const HcclB200MoeLayer *l, const char *api, std::initializer_list<void *const *> tables, MoeLocalLayer *out)
+// The tables of a call (rows: bf16 rows, moved in 16-byte vectors; words: experts and gates) and of its layer: an entry for
+// every rank, none of them null.
+static HcclResult moe_layer(Communicator *c, const HcclB200MoeLayer *l, const char *api, std::initializer_list<void *const *> rows,
+                            std::initializer_list<void *const *> words, MoeLocalLayer *out)
 {
     CHK_RET_LOG(!l, HCCL_E_PTR, "[EI0003] %s: layer is null", api);
-    for (void *const *t : tables) CHK_RET_LOG(!t, HCCL_E_PTR, "[EI0003] %s: null pointer", api);
+    for (void *const *t : rows) CHK_RET_LOG(!t, HCCL_E_PTR, "[EI0003] %s: null pointer", api);
+    for (void *const *t : words) CHK_RET_LOG(!t, HCCL_E_PTR, "[EI0003] %s: null pointer", api);
     CHK_RET_LOG(c->nlocal() != c->nranks() || l->nExperts > kMoeLocalMaxExperts, HCCL_E_NOT_SUPPORT,
                 "%s needs every rank of the communicator in this process on one GPU and at most %d experts", api, kMoeLocalMaxExperts);
     bool null = !l->scratch;
+    uintptr_t bits = 0, word_bits = 0;
     for (int r = 0; r < c->nranks(); ++r) {
         null = null || !l->rows[r] || !l->pos[r] || !l->dstRow[r] || !l->expertOffsets[r] || !l->recvRows[r] || !l->overflow[r];
-        for (void *const *t : tables) null = null || !t[r];
+        for (void *const *t : rows) { null = null || !t[r]; bits |= (uintptr_t)t[r]; }
+        for (void *const *t : words) { null = null || !t[r]; word_bits |= (uintptr_t)t[r]; }
     }
     CHK_RET_LOG(null, HCCL_E_PTR, "[EI0003] %s: null pointer in a table of the %d ranks", api, c->nranks());
+    CHK_RET_LOG((bits & 15) || (word_bits & 3), HCCL_E_PARA, "%s: rows must start on 16-byte boundaries, experts and gates on 4-byte ones", api);
     CHK_RET_LOG(c->transport() != TR_DEVICE, HCCL_E_NOT_SUPPORT, "%s needs the device transport", api);
     *out = MoeLocalLayer{l->tokens, l->capacityRows, c->nranks(), l->topk, l->hidden, l->nExperts, l->pos, l->dstRow, l->expertOffsets, l->recvRows,
                          l->overflow, l->scratch};
@@ -734,10 +740,11 @@ static HcclResult moe_layer(Communicator *c, const HcclB200MoeLayer *l, const ch
 HcclResult HcclB200MoeDispatchLocal(HcclComm comm, const HcclB200MoeLayer *layer, void *const *x, void *const *topkIdx, aclrtStream stream)
 {
     GET_COMM("HcclB200MoeDispatchLocal");
+    void *const *recv = layer ? layer->rows : nullptr;
     MoeLocalLayer l;
-    CHK_RET(moe_layer(c, layer, "HcclB200MoeDispatchLocal", {x, topkIdx}, &l));
+    CHK_RET(moe_layer(c, layer, "HcclB200MoeDispatchLocal", {recv, x}, {topkIdx}, &l));
     CHK_RET(c->ready());
-    return moe_local_dispatch(l, layer->rows, (const void *const *)x, (const int32_t *const *)topkIdx, stream);
+    return moe_local_dispatch(l, recv, (const void *const *)x, (const int32_t *const *)topkIdx, stream);
 }
 HcclResult HcclB200MoeCombineLocal(HcclComm comm, const HcclB200MoeLayer *layer, void *const *rows, void *const *topkIdx, void *const *gates,
                                    void *const *out, aclrtStream stream)
@@ -745,7 +752,7 @@ HcclResult HcclB200MoeCombineLocal(HcclComm comm, const HcclB200MoeLayer *layer,
     GET_COMM("HcclB200MoeCombineLocal");
     if (!rows && layer) rows = layer->rows;
     MoeLocalLayer l;
-    CHK_RET(moe_layer(c, layer, "HcclB200MoeCombineLocal", {rows, topkIdx, gates, out}, &l));
+    CHK_RET(moe_layer(c, layer, "HcclB200MoeCombineLocal", {rows, out}, {topkIdx, gates}, &l));
     CHK_RET(c->ready());
     return moe_local_combine(l, rows, (const int32_t *const *)topkIdx, (const float *const *)gates, out, stream);
 }

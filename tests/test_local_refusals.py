@@ -16,11 +16,12 @@ def pair():
     c.destroy()
 
 
-def moe_call(comm, missing=None, rank=1, entry="dispatch"):
-    """A dispatch or combine of the host communicator's ranks, with one entry of one table null: result code.  Complete tables
-    come as far as the check of the transport (the launches need a GPU)."""
+def moe_call(comm, missing=None, rank=1, entry="dispatch", instead=None):
+    """A dispatch or combine of the host communicator's ranks, with one entry of one table null (or moved by `instead` bytes):
+    result code.  Complete tables come as far as the check of the transport (the launches need a GPU)."""
     mem = C.create_string_buffer(64)
     at = (C.addressof(mem) + 31) // 32 * 32
+    odd = None if instead is None else at + instead
     y = L.MoeLayer(tokens=4, capacityRows=8, topk=2, hidden=8, nExperts=4, scratch=at)
     call = {n: (C.c_void_p * 2)(at, at) for n in ("x", "idx", "gates", "out", "given")}
     for n in PER_RANK:
@@ -29,9 +30,9 @@ def moe_call(comm, missing=None, rank=1, entry="dispatch"):
     if missing == "scratch":
         y.scratch = None
     elif missing in PER_RANK:
-        getattr(y, missing)[rank] = None
+        getattr(y, missing)[rank] = odd
     elif missing:
-        call[missing][rank] = None
+        call[missing][rank] = odd
     if entry == "dispatch":
         return L.lib().HcclB200MoeDispatchLocal(comm.handle, C.byref(y), call["x"], call["idx"], None)
     rows = call["given"] if missing == "given" else None
@@ -44,6 +45,17 @@ def test_moe_tables_with_a_null_entry(pair):
         for name in PER_RANK + ("scratch",) + tables:
             for rank in range(2):
                 assert moe_call(pair, name, rank, entry) == L.E_PTR, (entry, name, rank)
+
+
+def test_moe_rows_off_their_boundaries(pair):
+    """Rows move in 16-byte vectors, experts and gates in words: an address between is refused (32-byte vectors are a choice)."""
+    for entry, rows, words in (("dispatch", ("rows", "x"), ("idx",)), ("combine", ("rows", "out"), ("idx", "gates")), ("combine", ("given", "out"), ())):
+        for name in rows:
+            for off, want in ((2, L.E_PARA), (8, L.E_PARA), (16, L.E_NOT_SUPPORT)):
+                assert moe_call(pair, name, 1, entry, off) == want, (entry, name, off)
+        for name in words:
+            for off, want in ((2, L.E_PARA), (4, L.E_NOT_SUPPORT)):
+                assert moe_call(pair, name, 0, entry, off) == want, (entry, name, off)
 
 
 @pytest.mark.parametrize("nlocal,bad", [(1, None), (1, [None]), (2, [None, None])])
