@@ -8,8 +8,7 @@
 //   combine   the same split over the output rows, several tokens per CTA where top-k is small: eight expert rows in flight
 //             per thread, fp32 sum in k order, one rounding.
 //
-// Up to 65536 pairs over all ranks, the rows come from ONE cluster that counts in shared memory and registers; the dispatch
-// loads its activations and experts meanwhile.
+// Up to 65536 pairs over all ranks, the rows come from ONE cluster that counts in shared memory and registers.
 //
 // Bound: HBM for prefill batches (8192 tokens x 7168, top 8, one rank: dispatch 165 us at 6.4 TB/s, combine 156 us at 6.8 TB/s,
 // whole exchange 337 us, 468 us with a row read per expert, a launch per rank and step, and barriers), launches and L2 for
@@ -104,7 +103,7 @@ __global__ void __launch_bounds__(kCountThreads) moe_local_count_kernel(const __
     for (int e = threadIdx.x; e < E; e += kCountThreads) sh[e] = 0;
     __syncthreads();
     pdl_wait();
-    pdl_trigger();  // from here on the dispatch may read what this kernel found complete: activations and experts
+    pdl_trigger();
     for (int64_t i = i0 + threadIdx.x; i < i1; i += kCountThreads) {
         const int e = a.idx[r][i];
         a.pos[r][i] = e >= 0 && e < E ? atomicAdd(&sh[e], 1) : -1;
@@ -192,7 +191,7 @@ __global__ void __launch_bounds__(kCountThreads) moe_local_rows_kernel(const __g
     for (int i = threadIdx.x; i < a.p * E; i += kCountThreads) sh[i] = 0;
     __syncthreads();
     pdl_wait();
-    pdl_trigger();  // from here on the dispatch may read what this kernel found complete: activations and experts
+    pdl_trigger();
     int ex[kRowsRegs], ps[kRowsRegs], rk[kRowsRegs];
 #pragma unroll
     for (int k = 0; k < kRowsRegs; ++k) {
@@ -271,16 +270,14 @@ __global__ void __launch_bounds__(kDispatchThreads) moe_local_dispatch_kernel(co
     const int64_t t = a.nseg == 1 ? blockIdx.x : blockIdx.x / a.nseg;
     const int seg = (int)(blockIdx.x - t * a.nseg), per = (nvec + a.nseg - 1) / a.nseg, v1 = min(nvec, (seg + 1) * per);
     const V *src = (const V *)a.x[r] + t * nvec;
-    // the kernel before this one (rows or count) lets it start only after its own wait, and writes neither activations nor
-    // experts: they are loaded while it works
     const int v0 = seg * per + threadIdx.x;
+    // Nothing is read before this grid's own wait: only that makes what earlier kernels wrote (activations and experts among it)
+    // visible here, however early the kernel before this one triggered.
+    pdl_wait();
     V x[kPer];
 #pragma unroll
     for (int u = 0; u < kPer; ++u)
         if (v0 + u * nt < v1) x[u] = ld_row(src + v0 + u * nt);
-    int e0 = -1;
-    if (threadIdx.x < kRowBatch && (int)threadIdx.x < k) e0 = a.idx[r][t * k + threadIdx.x];
-    pdl_wait();
     for (int k0 = 0; k0 < k; k0 += kRowBatch) {
         if (k0) {
             __syncthreads();
@@ -292,7 +289,7 @@ __global__ void __launch_bounds__(kDispatchThreads) moe_local_dispatch_kernel(co
             V *d = nullptr;
             if (k0 + (int)threadIdx.x < k) {
                 const int64_t i = t * k + k0 + threadIdx.x;
-                const int known = kRows ? a.dst_row[r][i] : a.pos[r][i], e = k0 ? a.idx[r][i] : e0;
+                const int known = kRows ? a.dst_row[r][i] : a.pos[r][i], e = a.idx[r][i];
                 if (e >= 0 && e < a.n_experts) {
                     const int64_t row = kRows ? known : a.hist[((int64_t)r * a.nchunk + (uint32_t)i / (uint32_t)a.chunk) * a.n_experts + e] + known;
                     if (!kRows && seg == 0) a.dst_row[r][i] = (int32_t)row;

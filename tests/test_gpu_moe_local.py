@@ -80,3 +80,36 @@ def test_rows_beyond_the_capacity_are_dropped():
     assert bool((guard == 3).all())
     ex.close()
     c.destroy()
+
+
+@pytest.mark.parametrize("p,T,hidden,E,k", [(1, 128, 2048, 64, 8), (4, 128, 7168, 256, 8), (1, 8300, 64, 64, 8), (2, 4200, 512, 16, 8)])
+def test_inputs_rewritten_in_place(p, T, hidden, E, k):
+    """Activations and experts get new values at the same addresses, by kernels on the same stream right before every dispatch:
+    the rows that arrive are the new ones (numbered by one cluster, and through global memory).  No host wait in between."""
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    cfg = L.CommConfig.default()
+    cfg.hcclBufferSize = 2
+    c = H.Communicator.init_local(p, device=True, device_id=0, config=cfg)
+    ex = moe.MoEExchange(c, T, hidden, E, k, capacity_factor=float(p))
+    xs = [torch.zeros(T, hidden, device="cuda", dtype=torch.bfloat16) for _ in range(p)]
+    idx = [torch.zeros(T, k, device="cuda", dtype=torch.int32) for _ in range(p)]
+    kinds = [[(torch.randn(T, hidden, device="cuda").to(torch.bfloat16), moe.route(T, E, k, 11 + v, r)[0]) for r in range(p)] for v in range(3)]
+    good = torch.zeros(24, device="cuda", dtype=torch.bool)
+    El = E // p
+    torch.cuda.synchronize()
+    for it in range(good.numel()):
+        for r, (x, i) in enumerate(kinds[it % 3]):
+            torch.add(x, 0, out=xs[r])
+            idx[r].copy_(i)
+        ex.dispatch(xs if p > 1 else xs[0], idx if p > 1 else idx[0])
+        same = []
+        for r, (x, i) in enumerate(kinds[it % 3]):
+            rows = ex.dst_row[r].view(T, k).long()
+            got = torch.stack(ex.recv)[(i // El).long(), rows]
+            same.append((got == x[:, None, :]).all())
+        good[it] = torch.stack(same).all()
+    assert c.sync() == 0, c.describe_status()
+    assert bool(good.all()), good.nonzero().flatten().tolist()
+    ex.close()
+    c.destroy()
