@@ -689,7 +689,7 @@ HcclResult Communicator::run_collective_once(const OpRequest &rq)
     }
     if (is_v) sel_count = window;
     if (direct_applies(rq)) {
-        if (is_a2av) CHK_RET(a2av_check(rq));
+        if (is_a2av) CHK_RET(a2av_check(rq, true));
         int h0 = 0;
         size_t o0 = 0;
         const int label = p == 1 ? ALGO_SINGLE : (zc_candidate(rq) && registered_send(rq, &h0, &o0) ? ALGO_MESH_ZC : ALGO_DIRECT);
@@ -747,7 +747,7 @@ HcclResult Communicator::run_collective_once(const OpRequest &rq)
         HLOG_ERROR("NVLS algorithm requested but no multicast mapping exists on this communicator");
         return HCCL_E_NOT_SUPPORT;
     }
-    if (is_a2av) CHK_RET(a2av_check(rq));
+    if (is_a2av) CHK_RET(a2av_check(rq, false));
     CHK_RET(consistency_check(rq, sel.algo, use_zc ? ((uint64_t)zc[0].hin << 48) ^ zc[0].oin : 0, use_zc ? ((uint64_t)zc[0].hout << 48) ^ zc[0].oout : 0));
     if (sel.algo == ALGO_LL) {
         const bool blocked = rq.coll == COLL_REDUCE_SCATTER || rq.coll == COLL_ALLGATHER;  // count = one rank's block
@@ -1141,17 +1141,16 @@ HcclResult Communicator::consistency_check(const OpRequest &rq, int algo, uint64
 }
 
 // AlltoAllV / VC: what rank i sends to rank j must be what j expects from i (reference: alltoall_operator.cc:49-72 checks
-// the exchanged count matrix).  Virtual ranks hold the whole matrix; processes publish their two rows over the hub.  The
-// exchange costs a control-plane round trip, so by default only the first calls of a communicator are checked (the call
-// count is the same on every rank, so all ranks agree on which calls those are); HCCL_ALLTOALLV_CHECK=1 checks every
-// call, =0 none.
-HcclResult Communicator::a2av_check(const OpRequest &rq)
+// the exchanged count matrix).  Virtual ranks hold the whole matrix: every call is checked, a comparison of p x p words.
+// Processes publish their two rows over the hub.  That exchange costs a control-plane round trip, so by default only the first
+// calls of a communicator are checked (the call count is the same on every rank, so all ranks agree on which calls those are).
+// HCCL_ALLTOALLV_CHECK=1 checks every call, =0 none; `direct` is checked all the same, because its one copy per pair of
+// ranks trusts the sender's count, where the kernels that stage write no more than the receiver's.
+HcclResult Communicator::a2av_check(const OpRequest &rq, bool direct)
 {
     const int p = nranks_, nl = nlocal();
     const EnvConfig &env = env_config();
-    if (p == 1 || calibrating_ || env.a2av_check == 0) return HCCL_SUCCESS;
-    const uint64_t call = a2av_calls_++;
-    if (env.a2av_check < 0 && call >= 16) return HCCL_SUCCESS;
+    if (p == 1 || calibrating_ || (env.a2av_check == 0 && !direct)) return HCCL_SUCCESS;
     if (all_local_) {
         for (int i = 0; i < nl; ++i)
             for (int j = 0; j < nl; ++j) {
@@ -1161,6 +1160,8 @@ HcclResult Communicator::a2av_check(const OpRequest &rq)
             }
         return HCCL_SUCCESS;
     }
+    const uint64_t call = a2av_calls_++;
+    if (env.a2av_check < 0 && call >= 16) return HCCL_SUCCESS;
     std::string mine((const char *)rq.send_counts, (size_t)p * 8);
     mine.append((const char *)rq.recv_counts, (size_t)p * 8);
     std::vector<std::string> all;

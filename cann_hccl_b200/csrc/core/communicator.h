@@ -193,7 +193,7 @@ private:
     HcclResult tp_workspace(const std::string &key, size_t data_bytes, int M, void **ws_out);
     void tp_release_workspaces();
     int overlap_kind(const OpRequest &rq, int li) const;
-    HcclResult a2av_check(const OpRequest &rq);
+    HcclResult a2av_check(const OpRequest &rq, bool direct);
     HcclResult consistency_check(const OpRequest &rq, int algo, uint64_t zc_in = 0, uint64_t zc_out = 0);
     HcclResult maybe_retry(const OpRequest &rq, HcclResult failure, uint64_t op_index);
     // Device transport: the newest collective as it was issued (deep copy), so that a failure its kernel reports later,

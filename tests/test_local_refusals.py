@@ -83,3 +83,38 @@ def test_combine_before_any_dispatch():
     ex._topk = None
     with pytest.raises(RuntimeError):
         ex.combine(None)
+
+
+@pytest.mark.parametrize("device", [False, pytest.param(True, marks=pytest.mark.gpu)])
+def test_alltoallv_counts_are_compared_on_every_call(device):
+    """More calls than ranks of other processes would compare: a sender's count above the receiver's would run over the
+    receiver's next block."""
+    import numpy as np
+    if device:
+        torch = pytest.importorskip("torch")
+        if not torch.cuda.is_available():
+            pytest.skip("no GPU")
+    p, n = 3, 5
+    c = H.Communicator.init_local(p, device=device, device_id=0) if device else H.Communicator.init_local(p, device=False)
+    ins = [np.arange(p * n, dtype=np.float32) + 100 * r for r in range(p)]
+    outs = [np.full(p * (n + 1), -1, np.float32) for _ in range(p)]
+    if device:
+        ins, outs = [torch.from_numpy(x).cuda() for x in ins], [torch.from_numpy(x).cuda() for x in outs]
+    host = lambda x: x.cpu().numpy() if device else x
+    sc = np.full((p, p), n, np.uint64)
+    sd = np.tile(np.arange(p, dtype=np.uint64) * np.uint64(n), (p, 1))
+    rd = np.tile(np.arange(p, dtype=np.uint64) * np.uint64(n + 1), (p, 1))
+    for _ in range(20):
+        c.all_to_all_v(ins, sc, sd, outs, np.ascontiguousarray(sc.T), rd)
+    if device:
+        assert c.sync() == 0
+    before = [host(o).copy() for o in outs]
+    assert all(b[q * (n + 1)] == 100 * q + r * n and b[q * (n + 1) + n] == -1 for r, b in enumerate(before) for q in range(p))
+    for i, j, sent, expected in ((0, 2, n + 1, n), (2, 0, n, n + 1)):
+        m, want = sc.copy(), sc.T.copy()
+        m[i, j], want[j, i] = sent, expected
+        with pytest.raises(H.HcclError) as e:
+            c.all_to_all_v(ins, m, sd, outs, want, rd)
+        assert e.value.code == L.E_PARA
+    assert all(np.array_equal(b, host(o)) for b, o in zip(before, outs))
+    assert c.destroy() == L.SUCCESS
