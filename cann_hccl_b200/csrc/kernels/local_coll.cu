@@ -162,8 +162,8 @@ HcclResult launch_local_copy(LocalCopy &c, void *stream)
 // How a job lies over vectors of vb bytes: outputs first, the sources as they then come.
 static uint32_t layout_of(const LocalReduce &r, LocalReduceJob &j, uint32_t es, uint32_t vb)
 {
-    uint32_t differ = 0, shift = 0;
     const uintptr_t d0 = (uintptr_t)r.out[__builtin_ctz(j.mask)];
+    uint32_t differ = (uint32_t)d0 & (es - 1), shift = 0;  // an output that starts inside an element never meets a vector
     for (uint32_t m = j.mask; m; m &= m - 1) differ |= (uint32_t)((uintptr_t)r.out[__builtin_ctz(m)] ^ d0) & (vb - 1);
     j.head = (uint32_t)std::min<uint64_t>(j.count, ((vb - (d0 & (vb - 1))) & (vb - 1)) / es);
     j.nvec = (j.count - j.head) * es / vb;

@@ -30,6 +30,25 @@ __device__ __forceinline__ uint4 ld_shifted(const uint8_t *a)
     return s ? merge16(b[0], b[1], s) : b[0];
 }
 
+// One element of a buffer that need not start on a multiple of the element's size: byte by byte where it does not.
+template <class T> union ElemBytes { T e; uint8_t b[sizeof(T)]; __device__ ElemBytes() {} };
+template <class T> __device__ __forceinline__ T ld_elem(const uint8_t *p)
+{
+    if (((uintptr_t)p & (sizeof(T) - 1)) == 0) return *(const T *)p;
+    ElemBytes<T> v;
+#pragma unroll
+    for (int i = 0; i < (int)sizeof(T); ++i) v.b[i] = p[i];
+    return v.e;
+}
+template <class T> __device__ __forceinline__ void st_elem(uint8_t *p, T e)
+{
+    if (((uintptr_t)p & (sizeof(T) - 1)) == 0) { *(T *)p = e; return; }
+    ElemBytes<T> v;
+    v.e = e;
+#pragma unroll
+    for (int i = 0; i < (int)sizeof(T); ++i) p[i] = v.b[i];
+}
+
 // A vector is one load per source: 32 bytes where every address allows it, else 16.
 template <int VB> union Vec;
 template <> union Vec<16> { uint4 u; uint32_t w[4]; };
@@ -121,16 +140,17 @@ __global__ void __launch_bounds__(kLocalThreads) local_reduce_kernel(const __gri
         else if constexpr (VB == 16) local_reduce_tile<T, OP, NP, 16, 1, true>(a, j, tile);
         return;
     }
-    // one by one: what lies outside the vectors (a tile of its own), or everything when the outputs do not share an alignment
+    // one by one: what lies outside the vectors (a tile of its own), or everything when the outputs do not share an
+    // alignment or start inside an element
     const bool scalar = j.layout == LOCAL_SCALAR;
     const uint64_t vecs = scalar ? 0 : j.nvec, left = j.count - vecs * E;
     const uint64_t l0 = scalar ? (uint64_t)tile * a.tile_vecs * E : 0, l1 = scalar ? min(left, l0 + (uint64_t)a.tile_vecs * E) : left;
     for (uint64_t l = l0 + threadIdx.x; l < l1; l += kLocalThreads) {
         const uint64_t e = l < j.head ? l : vecs * E + l;
-        Acc acc = N::up(((const T *)(a.in[0] + j.off))[e]);
-        for (int q = 1; q < a.p; ++q) acc = red_op<OP>(acc, N::up(((const T *)(a.in[q] + j.off))[e]));
+        Acc acc = N::up(ld_elem<T>(a.in[0] + j.off + e * sizeof(T)));
+        for (int q = 1; q < a.p; ++q) acc = red_op<OP>(acc, N::up(ld_elem<T>(a.in[q] + j.off + e * sizeof(T))));
         const T r = N::down(acc);
-        for (uint32_t m = j.mask; m; m &= m - 1) ((T *)a.out[__ffs(m) - 1])[e] = r;
+        for (uint32_t m = j.mask; m; m &= m - 1) st_elem<T>(a.out[__ffs(m) - 1] + e * sizeof(T), r);
     }
 }
 

@@ -192,3 +192,39 @@ def test_variable_counts(comms):
         assert bool((rout[r][k:] == 9).all())
     c.barrier()
     assert c.sync() == 0
+
+
+class At:
+    """A buffer by its address: what a C caller passes."""
+
+    def __init__(self, t, off):
+        self.t, self.off = t, off
+
+    def data_ptr(self):
+        return self.t.data_ptr() + self.off
+
+
+@pytest.mark.parametrize("dtype,code", [(torch.float32, L.FP32), (torch.bfloat16, L.BFP16), (torch.float64, L.FP64)])
+@pytest.mark.parametrize("off_in,off_out", [((1, 1, 1), (0, 0, 0)), ((0, 0, 0), (1, 1, 1)), ((3, 1, 0), (0, 0, 0)), ((1, 2, 3), (5, 5, 5)), ((0, 1, 0), (1, 0, 3))])
+def test_reductions_of_buffers_inside_an_element(comms, dtype, code, off_in, off_out):
+    """Addresses that are no multiples of the element's size, on all ranks or on some: byte copies made them a matter of speed
+    on the kernels that stage."""
+    p = 3
+    c = comms(p)
+    es = torch.empty(0, dtype=dtype).element_size()
+    for n in (1, 37, 40_003):
+        ins = rnd(p, n * p, dtype, n)
+        mem = [torch.zeros(n * p * es + 64, device="cuda", dtype=torch.uint8) for _ in range(p)]
+        out = [torch.full((n * p * es + 64,), 9, device="cuda", dtype=torch.uint8) for _ in range(p)]
+        for m, x, o in zip(mem, ins, off_in):
+            m[16 + o:16 + o + n * p * es] = x.view(torch.uint8)
+        send, recv = [At(m, 16 + o) for m, o in zip(mem, off_in)], [At(m, 16 + o) for m, o in zip(out, off_out)]
+        for coll, count, mine in ((L.ALLREDUCE, n * p, lambda r: slice(0, n * p)), (L.REDUCE_SCATTER, n, lambda r: slice(r * n, (r + 1) * n))):
+            for m in out:
+                m.fill_(9)
+            c.collective(coll, send, recv, count, code, op=L.MAX)
+            done(c)
+            want = reduced(ins, L.MAX)
+            for r, (m, o) in enumerate(zip(out, off_out)):
+                assert torch.equal(m[16 + o:16 + o + count * es].clone().view(dtype).double(), want[mine(r)].double())
+                assert bool((m[:16 + o] == 9).all()) and bool((m[16 + o + count * es:] == 9).all())
