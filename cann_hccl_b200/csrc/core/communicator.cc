@@ -595,6 +595,16 @@ static void op_byte_ranges(const OpRequest &rq, int p, int rank, uint64_t *in_by
     *out_bytes = vout;
 }
 
+// A buffer that rank `rank` (local rank li) reads or writes is null.
+static bool null_buffer(const OpRequest &rq, int p, int rank, int li)
+{
+    uint64_t ib = 0, ob = 0;
+    op_byte_ranges(rq, p, rank, &ib, &ob);
+    if (rq.coll == COLL_ALLTOALLV || rq.coll == COLL_ALLTOALLVC)
+        for (int j = 0; j < p; ++j) { ib |= rq.send_counts[(size_t)li * p + j]; ob |= rq.recv_counts[(size_t)li * p + j]; }
+    return (ib && !(rq.in && rq.in[li])) || (ob && !(rq.out && rq.out[li]));
+}
+
 // 0: the buffers of local rank li are disjoint; 1: they overlap in the one form the op defines as "in place" (same
 // pointer, or the rank's own block at its position inside the larger buffer); 2: any other overlap.
 int Communicator::overlap_kind(const OpRequest &rq, int li) const
@@ -647,6 +657,8 @@ HcclResult Communicator::collective(const OpRequest &rq)
     // round for this op instead of giving up
     bool peer_failed = ready != HCCL_SUCCESS && remote_error_.load() == (uint32_t)ready && can_retry;
     if (ready != HCCL_SUCCESS && !peer_failed) return ready;
+    for (int li = 0; li < nlocal(); ++li)
+        CHK_RET_LOG(null_buffer(rq, nranks_, local_ranks_[li], li), HCCL_E_PTR, "[EI0003] %s: a buffer of rank %d is null", coll_name(rq.coll), local_ranks_[li]);
     for (int li = 0; li < nlocal(); ++li)
         CHK_RET_LOG(overlap_kind(rq, li) == 2, HCCL_E_PARA,
                     "%s: send and receive buffers of rank %d overlap in a way the operation does not define (in place means the same "

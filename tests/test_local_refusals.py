@@ -118,3 +118,35 @@ def test_alltoallv_counts_are_compared_on_every_call(device):
         assert e.value.code == L.E_PARA
     assert all(np.array_equal(b, host(o)) for b, o in zip(before, outs))
     assert c.destroy() == L.SUCCESS
+
+
+def test_collectives_with_a_null_buffer(pair):
+    """A rank without a buffer that the collective reads or writes is refused; one that the rank does not need may be missing."""
+    import numpy as np
+    n = 6
+    x, big = [np.ones(n, np.float32) for _ in range(2)], [np.zeros(2 * n, np.float32) for _ in range(2)]
+    need = {L.ALLREDUCE: (x, x), L.ALLGATHER: (x, big), L.REDUCE_SCATTER: (big, x), L.ALLTOALL: (x, big), L.BROADCAST: (x, x), L.REDUCE: (x, x),
+            L.SCATTER: (big, x), L.GATHER: (x, big)}
+    spare = {L.BROADCAST: {("send", 1), ("recv", 0)}, L.REDUCE: {("recv", 1)}, L.SCATTER: {("send", 1)}, L.GATHER: {("recv", 1)}}
+    for coll, (send, recv) in need.items():
+        for side in ("send", "recv"):
+            for rank in range(2):
+                if (side, rank) in spare.get(coll, ()):
+                    continue
+                s, r = list(send), [y.copy() for y in recv]
+                (s if side == "send" else r)[rank] = None
+                with pytest.raises(H.HcclError) as e:
+                    pair.collective(coll, s, r, 3, L.FP32, root=0)
+                assert e.value.code == L.E_PTR, (coll, side, rank)
+    out = [np.zeros(n, np.float32), None]                       # only the root receives
+    pair.reduce(x, out, 0)
+    assert np.array_equal(out[0], 2 * x[0])
+    c = np.array([[0, 2], [0, 0]], np.uint64)
+    d = np.zeros((2, 2), np.uint64)
+    got = [None, np.zeros(2, np.float32)]                       # rank 0 only sends, rank 1 only receives
+    pair.all_to_all_v([x[0], None], c, d, got, np.ascontiguousarray(c.T), d)
+    assert np.array_equal(got[1], x[0][:2])
+    for send, recv in (([None, x[0]], got), ([x[0], None], [x[0], None])):
+        with pytest.raises(H.HcclError) as e:
+            pair.collective(L.ALLTOALLV, send, recv, 0, L.FP32, rows=(c, d, np.ascontiguousarray(c.T), d))
+        assert e.value.code == L.E_PTR
