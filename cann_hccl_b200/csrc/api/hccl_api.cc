@@ -777,11 +777,19 @@ HcclResult HcclB200GemmLaunchCounts(uint64_t *single, uint64_t *pair)
     tp_gemm_launch_counts(single, pair);
     return HCCL_SUCCESS;
 }
+// A layer's operands and outputs: one for every local rank.
+static HcclResult check_layer(Communicator *c, void *const *a, void *const *b, void *const *out, const char *api)
+{
+    bool null = !a || !b || !out;
+    for (int i = 0; i < c->nlocal() && !null; ++i) null = !a[i] || !b[i] || !out[i];
+    CHK_RET_LOG(null, HCCL_E_PTR, "[EI0003] %s: null pointer", api);
+    return HCCL_SUCCESS;
+}
 HcclResult HcclB200AllGatherMatmulAct(HcclComm comm, void *const *xShards, void *const *weights, void *const *outs, int32_t M, int32_t N, int32_t K,
                                       int32_t act, aclrtStream stream)
 {
     GET_COMM("HcclB200AllGatherMatmul");
-    CHK_RET_LOG(!xShards || !weights || !outs, HCCL_E_PTR, "[EI0003] HcclB200AllGatherMatmul: null pointer");
+    CHK_RET(check_layer(c, xShards, weights, outs, "HcclB200AllGatherMatmul"));
     CHK_RET(check_act(act, "HcclB200AllGatherMatmulAct"));
     return c->tp_all_gather_matmul((const void *const *)xShards, (const void *const *)weights, outs, M, N, K, act, stream);
 }
@@ -794,7 +802,7 @@ HcclResult HcclB200MatmulReduceScatter(HcclComm comm, void *const *inputs, void 
                                        int32_t K, aclrtStream stream)
 {
     GET_COMM("HcclB200MatmulReduceScatter");
-    CHK_RET_LOG(!inputs || !weights || !outs, HCCL_E_PTR, "[EI0003] HcclB200MatmulReduceScatter: null pointer");
+    CHK_RET(check_layer(c, inputs, weights, outs, "HcclB200MatmulReduceScatter"));
     return c->tp_matmul_reduce_scatter((const void *const *)inputs, (const void *const *)weights, outs, M, N, K, stream);
 }
 HcclResult HcclB200GetKernelTrace(HcclComm comm, uint32_t localRank, uint64_t *out, size_t capWords, int32_t *nsteps)

@@ -76,6 +76,23 @@ def test_moe_call_path_refuses_none(nlocal, bad):
     assert L.fast.moe_combine(0, nlocal, 0, 0, good, good, good, 0) == L.E_PTR  # all buffers there: refused for the communicator
 
 
+def test_tensor_parallel_layers_with_a_null_entry(pair):
+    """Complete tables come as far as the check of the transport."""
+    mem = C.create_string_buffer(64)
+    at = C.addressof(mem)
+    lib = L.lib()
+    calls = {"gather": lambda t: lib.HcclB200AllGatherMatmul(pair.handle, *t, 256, 256, 64, None),
+             "gather_act": lambda t: lib.HcclB200AllGatherMatmulAct(pair.handle, *t, 256, 256, 64, 1, None),
+             "scatter": lambda t: lib.HcclB200MatmulReduceScatter(pair.handle, *t, 256, 256, 64, None)}
+    for name, call in calls.items():
+        assert call([(C.c_void_p * 2)(at, at) for _ in range(3)]) == L.E_NOT_SUPPORT
+        for table in range(3):
+            for rank in range(2):
+                t = [(C.c_void_p * 2)(at, at) for _ in range(3)]
+                t[table][rank] = None
+                assert call(t) == L.E_PTR, (name, table, rank)
+
+
 def test_combine_before_any_dispatch():
     pytest.importorskip("torch")
     from cann_hccl_b200.parallel import moe
