@@ -38,20 +38,20 @@ static int address(PyObject *x, void **out)
     return *out == NULL && PyErr_Occurred() ? -1 : 0;
 }
 
-/* one address per local rank; a rank that is alone may pass its buffer without a list */
+/* one address per local rank, from a list, a tuple or any other sequence (a stacked tensor gives one row per rank); a rank that is
+ * alone may pass its buffer without a list */
 static int addresses(PyObject *x, Py_ssize_t nlocal, void **out)
 {
-    const int list = PyList_Check(x), tuple = PyTuple_Check(x);
-    if (!list && !tuple) {
-        if (nlocal == 1) return address(x, out);
-        PyErr_SetString(PyExc_AssertionError, "need one buffer per local rank");
-        return -1;
-    }
-    const Py_ssize_t n = list ? PyList_GET_SIZE(x) : PyTuple_GET_SIZE(x);
+    if (!PyList_Check(x) && !PyTuple_Check(x) && nlocal == 1) return address(x, out);
+    const Py_ssize_t n = PyObject_Size(x);  /* before a long tensor is taken apart */
+    if (n < 0) return -1;
     if (n != nlocal) { PyErr_SetString(PyExc_AssertionError, "need one buffer per local rank"); return -1; }
-    for (Py_ssize_t i = 0; i < n; ++i)
-        if (address(list ? PyList_GET_ITEM(x, i) : PyTuple_GET_ITEM(x, i), out + i)) return -1;
-    return 0;
+    PyObject *seq = PySequence_Fast(x, "need one buffer per local rank");
+    if (!seq) return -1;
+    int rc = 0;
+    for (Py_ssize_t i = 0; i < nlocal && !rc; ++i) rc = address(PySequence_Fast_GET_ITEM(seq, i), out + i);
+    Py_DECREF(seq);
+    return rc;
 }
 
 /* the same where every rank has a buffer: None is refused */

@@ -1,4 +1,5 @@
-"""Calls that the paths for ranks of one process have to refuse on the host, before anything is launched."""
+"""Calls that the paths for ranks of one process have to refuse on the host, before anything is launched, and forms of a call that
+they have to go on taking."""
 import ctypes as C
 
 import pytest
@@ -167,3 +168,18 @@ def test_collectives_with_a_null_buffer(pair):
         with pytest.raises(H.HcclError) as e:
             pair.collective(L.ALLTOALLV, send, recv, 0, L.FP32, rows=(c, d, np.ascontiguousarray(c.T), d))
         assert e.value.code == L.E_PTR
+
+
+def test_buffers_as_rows_of_one_array(pair):
+    """One array with a row per rank is a list of buffers too; the number of rows has to be the number of ranks."""
+    import numpy as np
+    x, y = np.arange(10, dtype=np.float32).reshape(2, 5), np.zeros((2, 5), np.float32)
+    pair.collective(L.ALLREDUCE, x, y, 5, L.FP32)
+    assert np.array_equal(y, np.stack([x.sum(0)] * 2))
+    torch = pytest.importorskip("torch")
+    tx, ty = torch.arange(10.).reshape(2, 5), torch.zeros(2, 5)
+    pair.collective(L.ALLREDUCE, tx, ty, 5, L.FP32)
+    assert torch.equal(ty, tx.sum(0).repeat(2, 1))
+    for bad in (x[:1], [x[0]], (x[0], x[0], x[1])):
+        with pytest.raises(AssertionError):
+            pair.collective(L.ALLREDUCE, bad, y, 5, L.FP32)
