@@ -49,7 +49,12 @@ static int addresses(PyObject *x, Py_ssize_t nlocal, void **out)
     PyObject *seq = PySequence_Fast(x, "need one buffer per local rank");
     if (!seq) return -1;
     int rc = 0;
-    for (Py_ssize_t i = 0; i < nlocal && !rc; ++i) rc = address(PySequence_Fast_GET_ITEM(seq, i), out + i);
+    for (Py_ssize_t i = 0; i < nlocal && !rc; ++i) {
+        if (i >= PySequence_Fast_GET_SIZE(seq)) { PyErr_SetString(PyExc_AssertionError, "need one buffer per local rank"); rc = -1; break; }
+        PyObject *item = Py_NewRef(PySequence_Fast_GET_ITEM(seq, i));  /* asking it for its address runs Python code */
+        rc = address(item, out + i);
+        Py_DECREF(item);
+    }
     Py_DECREF(seq);
     return rc;
 }

@@ -183,3 +183,30 @@ def test_buffers_as_rows_of_one_array(pair):
     for bad in (x[:1], [x[0]], (x[0], x[0], x[1])):
         with pytest.raises(AssertionError):
             pair.collective(L.ALLREDUCE, bad, y, 5, L.FP32)
+
+
+def test_buffer_lists_that_are_not_what_they_say(pair):
+    """A list that shrinks while its buffers are asked for their addresses, a sequence whose length is not its items."""
+    import numpy as np
+    x = np.zeros(4, np.float32)
+
+    class Shrinks:
+        def __init__(self, of):
+            self.of = of
+
+        def data_ptr(self):
+            del self.of[1:]
+            return x.ctypes.data
+
+    class Short:
+        def __len__(self):
+            return 2
+
+        def __iter__(self):
+            return iter([x])
+
+    shrinking = []
+    shrinking += [Shrinks(shrinking), x]
+    for bad in (shrinking, Short()):
+        with pytest.raises(AssertionError):
+            pair.collective(L.ALLREDUCE, bad, [x, x.copy()], 4, L.FP32)
