@@ -36,6 +36,7 @@ enum AlgoId : int {
     ALGO_LL,            // AllReduce, small messages: data and flag travel together in 16-byte lines (device only)
     ALGO_MESH_ZC,       // AllReduce (two ranks) / ReduceScatter / AllGather on a registered send buffer: peers read it in place (kernels/pipe_coll.*)
     ALGO_DIRECT,        // AlltoAll family: parametric kernel, counts travel as launch arguments (kernels/a2av.cu; device only)
+    ALGO_LOCAL,         // every rank in this process on one GPU: one pass over memory, no staging (core/direct.cc; device only)
     ALGO_COUNT
 };
 const char *algo_name(int algo);

@@ -702,9 +702,7 @@ HcclResult Communicator::run_collective_once(const OpRequest &rq)
     if (is_v) sel_count = window;
     if (direct_applies(rq)) {
         if (is_a2av) CHK_RET(a2av_check(rq, true));
-        int h0 = 0;
-        size_t o0 = 0;
-        const int label = p == 1 ? ALGO_SINGLE : (zc_candidate(rq) && registered_send(rq, &h0, &o0) ? ALGO_MESH_ZC : ALGO_DIRECT);
+        const int label = p == 1 ? ALGO_SINGLE : ALGO_LOCAL;
         ++direct_ops_;
         for (int li = 0; li < nl; ++li) __atomic_store_n(&status_[li]->head, direct_ops_, __ATOMIC_RELAXED);
         HcclResult drc = run_direct(rq);
@@ -714,6 +712,7 @@ HcclResult Communicator::run_collective_once(const OpRequest &rq)
         record_trace(rq, label, 0, sel_count * es, now_us() - t0);
         return drc;
     }
+    CHK_RET_LOG(rq.algo == ALGO_LOCAL, HCCL_E_NOT_SUPPORT, "the direct kernels need every rank of the communicator in this process on one GPU");
     Selection sel = select(rq.coll, sel_count, rq.dtype, rq.redop);
     if (rq.algo != ALGO_AUTO) sel.algo = rq.algo;
     if (rq.nchan > 0) sel.nchan = rq.nchan;

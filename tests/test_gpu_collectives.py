@@ -409,8 +409,8 @@ def test_all_to_all_and_v(comms, p, algo):
 
 @pytest.mark.parametrize("p", [2, 3, 8])
 def test_all_to_all_v_parametric_kernel(comms, p):
-    """Auto selection on the device runs the parametric kernel: counts travel as launch arguments, so hundreds of distinct
-    count matrices build no plan and allocate nothing; blocks larger than a sub-slot go in acknowledged rounds."""
+    """The parametric kernel (the selector's choice for ranks of several processes): counts travel as launch arguments, so hundreds
+    of distinct count matrices build no plan and allocate nothing; blocks larger than a sub-slot go in acknowledged rounds."""
     import numpy as np
     c = comms(p)
     rng = np.random.default_rng(11)
@@ -429,7 +429,7 @@ def test_all_to_all_v_parametric_kernel(comms, p):
         for i in range(p):
             sd[i] = np.concatenate([[0], np.cumsum(m[i])[:-1]])
             rd[i] = np.concatenate([[0], np.cumsum(m[:, i])[:-1]])
-        c.all_to_all_v(vin, m, sd, vout, np.ascontiguousarray(m.T), rd)
+        c.all_to_all_v(vin, m, sd, vout, np.ascontiguousarray(m.T), rd, algo=L.ALGO_DIRECT)
         if it in (0, 60, 119):
             ok(c)
             assert c.trace()[-1]["algo"] == "direct"
@@ -446,8 +446,9 @@ def test_all_to_all_v_parametric_kernel(comms, p):
     n = 70_001
     ins = rnd(p, n * p, torch.float32, seed=8)
     outs = [torch.zeros(n * p, device="cuda") for _ in range(p)]
-    c.all_to_all(ins, outs)
+    c.all_to_all(ins, outs, algo=L.ALGO_DIRECT)
     ok(c)
+    assert c.trace()[-1]["algo"] == "direct"
     for r in range(p):
         for q in range(p):
             assert torch.equal(outs[r][q * n:(q + 1) * n], ins[q][r * n:(r + 1) * n])
@@ -466,26 +467,26 @@ def test_zero_copy_over_peer_mappings(comms, p):
     try:
         outs = [torch.zeros(n, device="cuda") for _ in range(p)]
         for _ in range(2):
-            c.reduce_scatter(zin, outs)
+            c.reduce_scatter(zin, outs, algo=L.ALGO_MESH_ZC)
         ok(c)
         assert c.trace()[-1]["algo"] == "mesh_zerocopy", c.trace()[-1]
         ref = ref_reduce(xs, L.SUM)
         for r, o in enumerate(outs):
             close(o, ref[r * n:(r + 1) * n], torch.float32, p)
         gout = [torch.zeros(n * p, device="cuda") for _ in range(p)]
-        c.all_gather([z[:n] for z in zin], gout)
+        c.all_gather([z[:n] for z in zin], gout, algo=L.ALGO_MESH_ZC)
         ok(c)
         assert c.trace()[-1]["algo"] == "mesh_zerocopy", c.trace()[-1]
         for o in gout:
             assert torch.equal(o, torch.cat([x[:n] for x in xs]))
         if p == 2:
             aouts = [torch.zeros(n * p, device="cuda") for _ in range(p)]
-            c.all_reduce(zin, aouts)
+            c.all_reduce(zin, aouts, algo=L.ALGO_MESH_ZC)
             ok(c)
             assert c.trace()[-1]["algo"] == "mesh_zerocopy", c.trace()[-1]
             for o in aouts:
                 close(o, ref, torch.float32, p)
-            c.all_reduce(zin, zin)   # in place would overwrite what the peer still reads: this form takes a staged path
+            c.all_reduce(zin, zin, nchan=2)   # in place would overwrite what the peer still reads: this form takes a staged path
             ok(c)
             assert c.trace()[-1]["algo"] != "mesh_zerocopy", c.trace()[-1]
             for z in zin:
@@ -516,6 +517,9 @@ def test_v_variants_barrier_sendrecv(comms):
     ref = ref_reduce(rin, L.SUM)
     for r in range(p):
         close(rout[r][:int(counts[r])], ref[int(displs[r]):int(displs[r] + counts[r])], torch.float32, p)
+    c.collective(L.BARRIER, None, None, 0, L.FP32, nchan=1)  # a CTA count: the barrier kernel
+    ok(c)
+    assert c.trace()[-1]["algo"] == "mesh", c.trace()[-1]
     c.barrier()
     ok(c)
     a = torch.randn(200_000, device="cuda")

@@ -58,7 +58,7 @@ def check(got, want, dtype, p):
     assert float((got.double() - want).abs().max()) <= p * p * eps
 
 
-def done(c, algo="direct"):
+def done(c, algo="local"):
     assert c.sync() == 0, c.describe_status()
     assert c.trace()[-1]["algo"] == algo, c.trace()[-1]
 

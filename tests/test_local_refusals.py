@@ -210,3 +210,15 @@ def test_buffer_lists_that_are_not_what_they_say(pair):
     for bad in (shrinking, Short()):
         with pytest.raises(AssertionError):
             pair.collective(L.ALLREDUCE, bad, [x, x.copy()], 4, L.FP32)
+
+
+def test_direct_kernels_by_name_need_one_gpu(pair):
+    """The algorithm of ranks that share a process and a GPU, asked for by its number: not on CPU ranks."""
+    import numpy as np
+    assert L.ALGO_NAMES[L.ALGO_LOCAL] == "local" and L.lib().HcclB200AlgoName(L.ALGO_LOCAL) == b"local"
+    x, y = [np.ones(4, np.float32) for _ in range(2)], [np.zeros(4, np.float32) for _ in range(2)]
+    with pytest.raises(H.HcclError) as e:
+        pair.all_reduce(x, y, algo=L.ALGO_LOCAL)
+    assert e.value.code == L.E_NOT_SUPPORT
+    pair.all_reduce(x, y)
+    assert pair.trace()[-1]["algo"] != "local" and np.array_equal(y[0], x[0] * 2)
