@@ -825,7 +825,8 @@ HcclResult HcclB200GetStatus(HcclComm comm, uint32_t localRank, HcclB200Status *
     CHK_RET_LOG(!st || localRank >= (uint32_t)c->nlocal(), HCCL_E_PARA, "HcclB200GetStatus: bad arguments");
     DevStatus *d = c->status((int)localRank);
     st->code = d->code; st->step = d->step; st->peer = d->peer; st->chan = d->chan;
-    st->expected = d->expected; st->seen = d->seen; st->seq = d->seq; st->head = d->head; st->tail = d->tail;
+    st->expected = d->expected; st->seen = d->seen; st->seq = d->seq;
+    st->head = d->head + c->direct_ops(); st->tail = d->tail + c->direct_ops();
     return HCCL_SUCCESS;
 }
 HcclResult HcclB200DescribeStatus(HcclComm comm, uint32_t localRank, char *text, size_t cap)
@@ -834,7 +835,7 @@ HcclResult HcclB200DescribeStatus(HcclComm comm, uint32_t localRank, char *text,
     CHK_RET_LOG(!text || localRank >= (uint32_t)c->nlocal(), HCCL_E_PARA, "HcclB200DescribeStatus: bad arguments");
     DevStatus *d = c->status((int)localRank);
     if (d->code == 0) snprintf(text, cap, "rank %d of %s: no error (ops started %llu, completed %llu)", c->ctx((int)localRank).rank,
-                               c->name().c_str(), (unsigned long long)d->head, (unsigned long long)d->tail);
+                               c->name().c_str(), (unsigned long long)(d->head + c->direct_ops()), (unsigned long long)(d->tail + c->direct_ops()));
     else
         snprintf(text, cap, "rank %d of %s: %s in op #%llu at step %d, channel %u, waiting for rank %d: flag expected >= 0x%llx "
                  "(op %llu, step value %llu) but saw 0x%llx (op %llu, step value %llu)",

@@ -703,9 +703,8 @@ HcclResult Communicator::run_collective_once(const OpRequest &rq)
     if (direct_applies(rq)) {
         if (is_a2av) CHK_RET(a2av_check(rq, true));
         const int label = p == 1 ? ALGO_SINGLE : ALGO_LOCAL;
-        ++direct_ops_;
-        for (int li = 0; li < nl; ++li) __atomic_store_n(&status_[li]->head, direct_ops_, __ATOMIC_RELAXED);
         HcclResult drc = run_direct(rq);
+        if (drc == HCCL_SUCCESS) direct_ops_.fetch_add(1, std::memory_order_relaxed);
         stats_.ops[rq.coll]++;
         stats_.bytes[rq.coll] += sel_count * es;
         stats_.algo_hist[label]++;

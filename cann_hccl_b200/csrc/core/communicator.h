@@ -103,6 +103,7 @@ public:
     CostModel &cost_model() { return model_; }
 
     HcclResult collective(const OpRequest &rq);
+    uint64_t direct_ops() const { return direct_ops_.load(std::memory_order_relaxed); }
     HcclResult ready() { std::lock_guard<std::mutex> lk(op_mu_); return check_ready(); }  // takes operations: not suspended, no failure on record
     // Send/Recv between two ranks.  Exactly one side per call on ordinary communicators; on all-local communicators
     // both sides are given and run together.
@@ -240,7 +241,7 @@ private:
     void *pinned_ = nullptr;               // host-mapped block holding status + abort words
     uint64_t p2p_slot_ = 0;
     uint64_t ll_seq_ = 0;                  // number of LL operations issued (tag and mailbox parity)
-    uint64_t direct_ops_ = 1ull << 62;     // op-execution id of the direct path (it consumes no plan sequence number)
+    std::atomic<uint64_t> direct_ops_{0};  // operations of the direct path (they consume no plan sequence number)
     bool ll_ok_ = false;
     uint64_t ll_two_shot_min_ = 256u << 10;  // from this size on the LL path of three and more ranks goes two-shot
     uint64_t ll_max_bytes() const;            // largest message the LL path takes on this communicator

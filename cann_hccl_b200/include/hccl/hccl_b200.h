@@ -60,7 +60,8 @@ extern HcclResult HcclB200StreamSync(HcclComm comm, aclrtStream stream);
 
 typedef struct HcclB200StatusDef {
     uint32_t code, step; int32_t peer; uint32_t chan;
-    uint64_t expected, seen, seq, head, tail;
+    uint64_t expected, seen, seq, head, tail;  /* head, tail: operations started and completed.  One whose kernels wait for nothing
+                                                * (every rank in this process on one GPU) counts as both once it is launched. */
 } HcclB200Status;
 /* ---- MoE expert-parallel dispatch / combine (kernels/moe_a2a.cu); bf16 rows, int32 expert ids, fp32 gates ---- */
 /* hist[e] = pairs routed to expert e, pos[i] = arrival index of pair i inside its expert group. */

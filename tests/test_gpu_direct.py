@@ -228,3 +228,21 @@ def test_reductions_of_buffers_inside_an_element(comms, dtype, code, off_in, off
             for r, (m, o) in enumerate(zip(out, off_out)):
                 assert torch.equal(m[16 + o:16 + o + count * es].clone().view(dtype).double(), want[mine(r)].double())
                 assert bool((m[:16 + o] == 9).all()) and bool((m[16 + o + count * es:] == 9).all())
+
+
+@pytest.mark.parametrize("p", [1, 2])
+def test_status_counts_operations(p):
+    """Operations started and completed, on a communicator that has run nothing else and after an operation on staged kernels."""
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    c = H.Communicator.init_local(p, device=True, device_id=0)
+    x, y = [torch.ones(1 << 12, device="cuda") for _ in range(p)], [torch.zeros(1 << 12, device="cuda") for _ in range(p)]
+    for n in (1, 2, 3):
+        c.all_reduce(x, y)
+        assert c.sync() == 0
+        st = c.status(p - 1)
+        assert (st.head, st.tail) == (n, n) and "ops started %d, completed %d)" % (n, n) in c.describe_status(p - 1)
+    c.all_reduce(x, y, nchan=2, algo=L.ALGO_MESH if p > 1 else L.ALGO_SINGLE)
+    c.all_reduce(x, y)
+    assert c.sync() == 0 and c.status(0).head == 5
+    c.destroy()
