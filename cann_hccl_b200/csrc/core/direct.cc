@@ -11,13 +11,13 @@ namespace hcclb {
 
 // The choice for such communicators where nothing else is asked for.  Another algorithm (that of the parametric AlltoAll and of
 // the peers' registered buffers included), a CTA count or an execution mode that the caller or the environment asks for keeps
-// the staged kernels, which is how those are tested on one GPU.
+// the staged kernels, which is how those are tested on one GPU; so do in-kernel timestamps (HCCL_KERNEL_TRACE), which only those write.
 bool Communicator::direct_applies(const OpRequest &rq) const
 {
     if (settings_.transport != TR_DEVICE || nlocal() != nranks_ || calibrating_) return false;
     if (rq.algo == ALGO_LOCAL) return true;
     const EnvConfig &env = env_config();
-    if (rq.algo != ALGO_AUTO || rq.nchan > 0 || env.channels > 0) return false;
+    if (rq.algo != ALGO_AUTO || rq.nchan > 0 || env.channels > 0 || dev_trace_) return false;
     if ((settings_.expansion_mode ? settings_.expansion_mode : env.expansion_mode) == 1) return false;
     return env.algo.empty() || forced_algo_for(env, rq.coll).empty();
 }

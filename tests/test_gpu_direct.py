@@ -1,5 +1,7 @@
 """Direct collectives of communicators that hold every rank in this process on one GPU (algorithm left to the selector),
 against a plain PyTorch reference: sizes around vectors and tiles, every alignment, in-place forms."""
+import ctypes as C
+
 import pytest
 
 torch = pytest.importorskip("torch")
@@ -245,4 +247,22 @@ def test_status_counts_operations(p):
     c.all_reduce(x, y, nchan=2, algo=L.ALGO_MESH if p > 1 else L.ALGO_SINGLE)
     c.all_reduce(x, y)
     assert c.sync() == 0 and c.status(0).head == 5
+    c.destroy()
+
+
+@pytest.mark.parametrize("p", [1, 3])
+def test_kernel_trace_is_filled(p, monkeypatch):
+    """HCCL_KERNEL_TRACE at the communicator's creation: the selector's choice writes in-kernel timestamps."""
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    monkeypatch.setenv("HCCL_KERNEL_TRACE", "1")
+    c = H.Communicator.init_local(p, device=True, device_id=0)
+    x, y = [torch.ones(3 << 20, device="cuda") for _ in range(p)], [torch.zeros(3 << 20, device="cuda") for _ in range(p)]
+    c.all_reduce(x, y)
+    assert c.sync() == 0 and bool((y[0] == p).all())
+    words = (C.c_uint64 * 16)()
+    assert L.lib().HcclB200GetKernelTrace(c.handle, 0, words, 16, None) == 0
+    assert 0 < words[0] < 2 ** 64 - 1 and any(words[1:])
+    c.all_reduce(x, y, algo=L.ALGO_LOCAL)
+    assert c.sync() == 0 and bool((y[p - 1] == p).all())
     c.destroy()
