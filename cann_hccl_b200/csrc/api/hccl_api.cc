@@ -743,7 +743,7 @@ HcclResult HcclB200MoeDispatchLocal(HcclComm comm, const HcclB200MoeLayer *layer
     void *const *recv = layer ? layer->rows : nullptr;
     MoeLocalLayer l;
     CHK_RET(moe_layer(c, layer, "HcclB200MoeDispatchLocal", {recv, x}, {topkIdx}, &l));
-    CHK_RET(c->ready());
+    CHK_RET(c->begin_launches(2));  // rows or count, dispatch
     return moe_local_dispatch(l, recv, (const void *const *)x, (const int32_t *const *)topkIdx, stream);
 }
 HcclResult HcclB200MoeCombineLocal(HcclComm comm, const HcclB200MoeLayer *layer, void *const *rows, void *const *topkIdx, void *const *gates,
@@ -753,7 +753,7 @@ HcclResult HcclB200MoeCombineLocal(HcclComm comm, const HcclB200MoeLayer *layer,
     if (!rows && layer) rows = layer->rows;
     MoeLocalLayer l;
     CHK_RET(moe_layer(c, layer, "HcclB200MoeCombineLocal", {rows, out}, {topkIdx, gates}, &l));
-    CHK_RET(c->ready());
+    CHK_RET(c->begin_launches(1));
     return moe_local_combine(l, rows, (const int32_t *const *)topkIdx, (const float *const *)gates, out, stream);
 }
 static HcclResult check_act(int32_t act, const char *api)

@@ -104,7 +104,15 @@ public:
 
     HcclResult collective(const OpRequest &rq);
     uint64_t direct_ops() const { return direct_ops_.load(std::memory_order_relaxed); }
-    HcclResult ready() { std::lock_guard<std::mutex> lk(op_mu_); return check_ready(); }  // takes operations: not suspended, no failure on record
+    // For kernels that other layers launch on this communicator's behalf: HCCL_SUCCESS while it takes operations (not suspended, no
+    // failure on record), and the launches are counted.
+    HcclResult begin_launches(int n)
+    {
+        std::lock_guard<std::mutex> lk(op_mu_);
+        HcclResult rc = check_ready();
+        if (rc == HCCL_SUCCESS) stats_.launches += (uint64_t)n;
+        return rc;
+    }
     // Send/Recv between two ranks.  Exactly one side per call on ordinary communicators; on all-local communicators
     // both sides are given and run together.
     HcclResult send(const void *buf, uint64_t count, int dtype, int dest, void *stream);

@@ -27,8 +27,8 @@ HcclResult Communicator::run_direct(const OpRequest &rq)
     const int p = nranks_;
     const uint64_t es = (uint64_t)dtype_size(rq.dtype), n = rq.count;
     const uint32_t all = (1u << p) - 1u;
-    stats_.launches++;
     if (rq.coll == COLL_BARRIER) return HCCL_SUCCESS;  // one stream carries every rank: stream order is the barrier
+    stats_.launches++;
 
     const bool reduces = rq.coll == COLL_ALLREDUCE || rq.coll == COLL_REDUCE || rq.coll == COLL_REDUCE_SCATTER || rq.coll == COLL_REDUCE_SCATTER_V;
     if (reduces && p > 1) {

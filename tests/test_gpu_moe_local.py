@@ -31,6 +31,7 @@ def test_exchange(p, T, hidden, E, k, per_rank):
     xs = [torch.randn(T, hidden, device="cuda", generator=g).to(torch.bfloat16) for _ in range(p)]
     idx, gates = map(list, zip(*[moe.route(T, E, k, 7, r) for r in range(p)]))
     idx[0][0, 0] = -1                                            # a slot without an expert is skipped
+    launches = c.stats()["launches"]
     for _ in range(2):                                            # the second call finds the scratch as the first left it
         ex.dispatch(xs if p > 1 else xs[0], idx if p > 1 else idx[0])
         assert c.sync() == 0, c.describe_status()
@@ -57,6 +58,8 @@ def test_exchange(p, T, hidden, E, k, per_rank):
             tol = 2.0 ** -8 * (1 + (k - 1) // 8)
             assert bool(((same[r].float() - want).abs() <= tol * xs[r].float().abs() + 1e-6).all())
             assert torch.equal(outs[r], -same[r])
+    # two dispatches of two launches and four combines of one; per rank: an all-gather (or its direct copy) and barriers each time
+    assert c.stats()["launches"] == launches + 8 if not per_rank else c.stats()["launches"] > launches
     ex.close()
     c.destroy()
 
