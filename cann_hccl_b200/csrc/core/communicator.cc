@@ -452,6 +452,26 @@ HcclResult Communicator::check_ready()
 
 Selection Communicator::select(int coll, uint64_t count, int dtype, int redop) const
 {
+    if (nranks_ == 1 || !direct_default(coll)) return select_staged(coll, count, dtype, redop);
+    // every input byte read once, every output byte written once, over all ranks; gamma counts a byte that is read and written once
+    const double n = (double)count * dtype_size(dtype), p = nranks_;
+    double touched = 2 * p * n;
+    switch (coll) {
+        case COLL_BARRIER: touched = 0; break;
+        case COLL_BROADCAST: touched = p * n; break;
+        case COLL_REDUCE: touched = (p + 1) * n; break;
+        case COLL_REDUCE_SCATTER: case COLL_REDUCE_SCATTER_V: case COLL_ALLGATHER: case COLL_ALLGATHER_V: touched = (p * p + p) * n; break;
+        default: break;
+    }
+    Selection s;
+    s.algo = ALGO_LOCAL;
+    s.nchan = 0;  // a grid of its own
+    s.est_us = model_.launch_us + touched / 2 / (model_.gamma_gbps * 1e3);
+    return s;
+}
+
+Selection Communicator::select_staged(int coll, uint64_t count, int dtype, int redop) const
+{
     const EnvConfig &env = env_config();
     SelectInput si;
     si.coll = coll;
@@ -712,7 +732,7 @@ HcclResult Communicator::run_collective_once(const OpRequest &rq)
         return drc;
     }
     CHK_RET_LOG(rq.algo == ALGO_LOCAL, HCCL_E_NOT_SUPPORT, "the direct kernels need every rank of the communicator in this process on one GPU");
-    Selection sel = select(rq.coll, sel_count, rq.dtype, rq.redop);
+    Selection sel = select_staged(rq.coll, sel_count, rq.dtype, rq.redop);
     if (rq.algo != ALGO_AUTO) sel.algo = rq.algo;
     if (rq.nchan > 0) sel.nchan = rq.nchan;
     if (p == 1) sel.algo = ALGO_SINGLE;

@@ -160,6 +160,8 @@ public:
     HcclResult tp_matmul_reduce_scatter(const void *const *h, const void *const *w, void *const *out, int M, int N, int K, void *stream);
     // Selection only (no execution).
     Selection select(int coll, uint64_t count, int dtype, int redop) const;
+    // The same among the kernels that stage: what runs where the direct path is not taken.
+    Selection select_staged(int coll, uint64_t count, int dtype, int redop) const;
     const CommStats &stats() const { return stats_; }
     std::vector<TraceRecord> trace_snapshot();
     std::string stats_json();
@@ -193,6 +195,7 @@ private:
     HcclResult run_ll_allreduce(const OpRequest &rq);
     HcclResult run_pipe(const OpRequest &rq, bool want_mc, int zc_handle = 0, size_t zc_off = 0);
     HcclResult run_a2av(const OpRequest &rq);
+    bool direct_default(int coll) const;             // for requests that ask for nothing else
     bool direct_applies(const OpRequest &rq) const;  // core/direct.cc: all ranks in this process on one GPU
     HcclResult run_direct(const OpRequest &rq);
     bool zc_candidate(const OpRequest &rq) const;

@@ -14,12 +14,17 @@ namespace hcclb {
 // the staged kernels, which is how those are tested on one GPU; so do in-kernel timestamps (HCCL_KERNEL_TRACE), which only those write.
 bool Communicator::direct_applies(const OpRequest &rq) const
 {
-    if (settings_.transport != TR_DEVICE || nlocal() != nranks_ || calibrating_) return false;
-    if (rq.algo == ALGO_LOCAL) return true;
+    if (calibrating_) return false;  // measures the staged kernels, which requests of those kinds choose among
+    if (rq.algo == ALGO_LOCAL) return settings_.transport == TR_DEVICE && nlocal() == nranks_;
+    return rq.algo == ALGO_AUTO && rq.nchan <= 0 && direct_default(rq.coll);
+}
+
+bool Communicator::direct_default(int coll) const
+{
     const EnvConfig &env = env_config();
-    if (rq.algo != ALGO_AUTO || rq.nchan > 0 || env.channels > 0 || dev_trace_) return false;
+    if (settings_.transport != TR_DEVICE || nlocal() != nranks_ || env.channels > 0 || dev_trace_) return false;
     if ((settings_.expansion_mode ? settings_.expansion_mode : env.expansion_mode) == 1) return false;
-    return env.algo.empty() || forced_algo_for(env, rq.coll).empty();
+    return env.algo.empty() || forced_algo_for(env, coll).empty();
 }
 
 HcclResult Communicator::run_direct(const OpRequest &rq)

@@ -266,3 +266,18 @@ def test_kernel_trace_is_filled(p, monkeypatch):
     c.all_reduce(x, y, algo=L.ALGO_LOCAL)
     assert c.sync() == 0 and bool((y[p - 1] == p).all())
     c.destroy()
+
+
+def test_select_names_what_runs(comms):
+    """The selector's answer without a run: the direct kernels on ranks of one process, the single-rank copy for a lone rank."""
+    c = comms(4)
+    x, y = [torch.ones(1 << 18, device="cuda") for _ in range(4)], [torch.zeros(1 << 20, device="cuda") for _ in range(4)]
+    c.all_reduce(x, [t[:1 << 18] for t in y])
+    done(c, c.select(L.ALLREDUCE, 1 << 18, L.FP32)[0])
+    c.all_gather(x, y)
+    done(c, c.select(L.ALLGATHER, 1 << 18, L.FP32)[0])
+    times = [c.select(L.ALLREDUCE, n, L.FP32)[2] for n in (1 << 10, 1 << 20, 1 << 24)]
+    assert 0 < times[0] < times[1] < times[2]
+    one = comms(1)
+    one.all_reduce(x[:1], [y[0][:1 << 18]])
+    done(one, one.select(L.ALLREDUCE, 1 << 18, L.FP32)[0])
