@@ -1,6 +1,7 @@
 """ctypes binding of libhccl_b200.so (the C API of include/hccl/hccl.h and hccl_b200.h)."""
 import ctypes as C
 import os
+import warnings
 from importlib.machinery import ExtensionFileLoader
 from importlib.util import module_from_spec, spec_from_loader
 
@@ -90,7 +91,7 @@ class MoeLayer(C.Structure):
 
 
 _lib = None
-fast = None  # csrc/python/fastcall.c, bound to the loaded library
+fast = None  # csrc/python/fastcall.c, bound to the loaded library (or _calls.py in its place)
 
 
 def _nccl_path():
@@ -110,8 +111,8 @@ def lib():
     global _lib, fast
     if _lib is not None:
         return _lib
-    from . import build as _build
-    if not os.path.exists(LIB_PATH) or not os.path.exists(_build.fastcall_path()):
+    if not os.path.exists(LIB_PATH):
+        from . import build as _build
         _build.build()
     if "HCCL_NCCL_LIB" not in os.environ:
         p = _nccl_path()
@@ -231,12 +232,28 @@ def lib():
     L.HcclB200AlgoName.restype = C.c_char_p
     L.HcclGetCommConfigCapability.argtypes = []
     L.HcclGetCommConfigCapability.restype = C.c_uint32
-    loader = ExtensionFileLoader("_fastcall", _build.fastcall_path())
-    fast = module_from_spec(spec_from_loader("_fastcall", loader))
-    loader.exec_module(fast)
-    fast.bind(*[C.cast(f, vp).value for f in (L.HcclB200Collective, L.HcclB200MoeDispatchLocal, L.HcclB200MoeCombineLocal)])
+    fast = _load_fast(L)
     _lib = L
     return L
+
+
+def _load_fast(L):
+    """The call path: the extension of this interpreter, compiled when it is missing (the library may come from elsewhere), or the
+    same calls through ctypes where it cannot be."""
+    from . import build as _build
+    path = _build.fastcall_path()
+    try:
+        if not os.path.exists(path):
+            _build.build_fastcall()
+        loader = ExtensionFileLoader("_fastcall", path)
+        m = module_from_spec(spec_from_loader("_fastcall", loader))
+        loader.exec_module(m)
+    except (OSError, ImportError, RuntimeError) as e:
+        from ._calls import Calls
+        warnings.warn("calls go through ctypes, which costs several microseconds each: %s" % (str(e).splitlines() or [type(e).__name__])[0])
+        return Calls(L)
+    m.bind(*[C.cast(f, C.c_void_p).value for f in (L.HcclB200Collective, L.HcclB200MoeDispatchLocal, L.HcclB200MoeCombineLocal)])
+    return m
 
 
 class HcclError(RuntimeError):

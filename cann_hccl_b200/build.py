@@ -73,20 +73,26 @@ def lib_path(sanitize=None):
 
 
 def fastcall_path():
-    """The call path of the Python layer (csrc/python/fastcall.c), an extension module of the running interpreter."""
-    return os.path.join(LIB, "_fastcall.so")
+    """The call path of the Python layer (csrc/python/fastcall.c), an extension module.  Its name carries the tag of the interpreter
+    that it is built for, so that another one never loads it."""
+    return os.path.join(LIB, "_fastcall" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 
-def _build_fastcall(force, verbose):
+def build_fastcall(force=False, verbose=False):
+    """Compile the extension for the running interpreter (a C compiler and its headers are all it takes).  The file appears in one
+    step: several ranks may find it missing at once."""
     src, out = os.path.join(CSRC, "python", "fastcall.c"), fastcall_path()
     if not force and os.path.exists(out) and os.path.getmtime(out) >= max(os.path.getmtime(src), _newest_header()):
         return
-    cmd = ["gcc", "-O2", "-g", "-fPIC", "-shared", "-std=c11", "-Wall", "-I" + INC, "-I" + sysconfig.get_paths()["include"], src, "-o", out]
+    os.makedirs(LIB, exist_ok=True)
+    part = "%s.%d" % (out, os.getpid())
+    cmd = ["gcc", "-O2", "-g", "-fPIC", "-shared", "-std=c11", "-Wall", "-I" + INC, "-I" + sysconfig.get_paths()["include"], src, "-o", part]
     if verbose:
         print(" ".join(cmd), flush=True)
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("compile failed: %s\n%s\n%s" % (" ".join(cmd), r.stdout, r.stderr))
+    os.replace(part, out)
 
 
 def build(force=False, verbose=False, sanitize=None):
@@ -102,7 +108,7 @@ def build(force=False, verbose=False, sanitize=None):
         san_link = ["-Xcompiler", flag]
     os.makedirs(OBJ, exist_ok=True)
     os.makedirs(LIB, exist_ok=True)
-    _build_fastcall(force, verbose)
+    build_fastcall(force, verbose)
     hdr = _newest_header()
     jobs, objs = [], []
     for src in _sources():
