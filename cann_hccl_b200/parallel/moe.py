@@ -64,6 +64,7 @@ class MoEExchange:
                 getattr(y, name)[r] = t.data_ptr()
         self._out_rows = (C.c_void_p * 16)(*[t.data_ptr() for t in self.expert_out])
         self._layer_ptr, self._out_ptr = C.addressof(y), C.addressof(self._out_rows)
+        torch.cuda.current_stream(device).synchronize()  # the scratch is zero whatever stream the first dispatch runs on
         return y
 
     def _l(self, x):

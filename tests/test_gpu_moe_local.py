@@ -116,3 +116,28 @@ def test_inputs_rewritten_in_place(p, T, hidden, E, k):
     assert bool(good.all()), good.nonzero().flatten().tolist()
     ex.close()
     c.destroy()
+
+
+def test_first_dispatch_on_another_stream():
+    """The exchange is made while its stream is busy and used on another one at once: the numbering of more pairs than one cluster
+    takes needs the scratch zero from the start."""
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    T, hidden, E, k = 8300, 64, 64, 8
+    c = H.Communicator.init_root(1, H.Communicator.get_root_info(), 0, device=True)
+    x = torch.randn(T, hidden, device="cuda").to(torch.bfloat16)
+    idx, gates = moe.route(T, E, k, 5, 0)
+    side = torch.cuda.Stream()
+    words = L.lib().HcclB200MoeScratchBytes(1, T, k, E) // 4
+    torch.full((words,), 7, device="cuda", dtype=torch.int32)  # what the allocator hands out next is not zero by chance
+    torch.cuda.synchronize()
+    torch.cuda._sleep(50_000_000)
+    ex = moe.MoEExchange(c, T, hidden, E, k)
+    with torch.cuda.stream(side):
+        ex.dispatch(x, idx)
+        out = ex.combine(gates, source="recv")
+    side.synchronize()
+    assert int(ex.recv_rows[0]) == T * k and torch.equal(ex.recv[0][ex.dst_row[0].view(T, k).long()], x[:, None].expand(T, k, hidden))
+    assert bool(((out.float() - x.float()).abs() <= 2.0 ** -8 * x.float().abs() + 1e-6).all())
+    ex.close()
+    c.destroy()
