@@ -71,6 +71,8 @@ class MoEExchange:
         return list(x) if isinstance(x, (list, tuple)) else [x]
 
     def dispatch(self, x, topk_idx, variant="mesh"):
+        if self.recv is None:
+            raise RuntimeError("dispatch() on a closed exchange")
         xs, idx = self._l(x), self._l(topk_idx)
         if self._layer is not None:  # no links between the ranks: the variants, which order the traffic on them, are one
             for t, i in zip(xs, idx):
@@ -129,7 +131,7 @@ class MoEExchange:
         return outs[0] if self.nl == 1 else outs
 
     def close(self):
-        self.recv = self.expert_out = None
+        self.recv = self.expert_out = self._topk = None  # nothing reaches the memory given back here
         self.comm.mem_free(self.h_recv)
         self.comm.mem_free(self.h_out)
 

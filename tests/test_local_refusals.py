@@ -103,6 +103,27 @@ def test_combine_before_any_dispatch():
         ex.combine(None)
 
 
+def test_closed_exchange():
+    pytest.importorskip("torch")
+    from cann_hccl_b200.parallel import moe
+
+    class Memory:
+        freed = []
+
+        def mem_free(self, handle):
+            self.freed.append(handle)
+
+    ex = object.__new__(moe.MoEExchange)
+    ex.comm, ex.h_recv, ex.h_out, ex._topk = Memory(), 1, 2, [object()]
+    ex.recv = ex.expert_out = [object()]
+    ex.close()
+    assert ex.comm.freed == [1, 2]
+    with pytest.raises(RuntimeError):
+        ex.dispatch(None, None)
+    with pytest.raises(RuntimeError):
+        ex.combine(None)
+
+
 @pytest.mark.parametrize("device", [False, pytest.param(True, marks=pytest.mark.gpu)])
 def test_alltoallv_counts_are_compared_on_every_call(device):
     """More calls than ranks of other processes would compare: a sender's count above the receiver's would run over the
