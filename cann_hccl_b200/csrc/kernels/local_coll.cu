@@ -7,34 +7,34 @@
 
 namespace hcclb {
 
-const void *local_kernel_i8(int op, int p, bool wide);
-const void *local_kernel_u8(int op, int p, bool wide);
-const void *local_kernel_i16(int op, int p, bool wide);
-const void *local_kernel_u16(int op, int p, bool wide);
-const void *local_kernel_i32(int op, int p, bool wide);
-const void *local_kernel_u32(int op, int p, bool wide);
-const void *local_kernel_i64(int op, int p, bool wide);
-const void *local_kernel_u64(int op, int p, bool wide);
-const void *local_kernel_f32(int op, int p, bool wide);
-const void *local_kernel_f64(int op, int p, bool wide);
-const void *local_kernel_f16(int op, int p, bool wide);
-const void *local_kernel_bf16(int op, int p, bool wide);
+const void *local_kernel_i8(int op, int p, bool wide, bool bytes);
+const void *local_kernel_u8(int op, int p, bool wide, bool bytes);
+const void *local_kernel_i16(int op, int p, bool wide, bool bytes);
+const void *local_kernel_u16(int op, int p, bool wide, bool bytes);
+const void *local_kernel_i32(int op, int p, bool wide, bool bytes);
+const void *local_kernel_u32(int op, int p, bool wide, bool bytes);
+const void *local_kernel_i64(int op, int p, bool wide, bool bytes);
+const void *local_kernel_u64(int op, int p, bool wide, bool bytes);
+const void *local_kernel_f32(int op, int p, bool wide, bool bytes);
+const void *local_kernel_f64(int op, int p, bool wide, bool bytes);
+const void *local_kernel_f16(int op, int p, bool wide, bool bytes);
+const void *local_kernel_bf16(int op, int p, bool wide, bool bytes);
 
-static const void *local_kernel_for(int dtype, int op, int p, bool wide)
+static const void *local_kernel_for(int dtype, int op, int p, bool wide, bool bytes)
 {
     switch (dtype) {
-        case HCCL_DATA_TYPE_INT8: return local_kernel_i8(op, p, wide);
-        case HCCL_DATA_TYPE_UINT8: return local_kernel_u8(op, p, wide);
-        case HCCL_DATA_TYPE_INT16: return local_kernel_i16(op, p, wide);
-        case HCCL_DATA_TYPE_UINT16: return local_kernel_u16(op, p, wide);
-        case HCCL_DATA_TYPE_INT32: return local_kernel_i32(op, p, wide);
-        case HCCL_DATA_TYPE_UINT32: return local_kernel_u32(op, p, wide);
-        case HCCL_DATA_TYPE_INT64: return local_kernel_i64(op, p, wide);
-        case HCCL_DATA_TYPE_UINT64: return local_kernel_u64(op, p, wide);
-        case HCCL_DATA_TYPE_FP32: return local_kernel_f32(op, p, wide);
-        case HCCL_DATA_TYPE_FP64: return local_kernel_f64(op, p, wide);
-        case HCCL_DATA_TYPE_FP16: return local_kernel_f16(op, p, wide);
-        case HCCL_DATA_TYPE_BFP16: return local_kernel_bf16(op, p, wide);
+        case HCCL_DATA_TYPE_INT8: return local_kernel_i8(op, p, wide, bytes);
+        case HCCL_DATA_TYPE_UINT8: return local_kernel_u8(op, p, wide, bytes);
+        case HCCL_DATA_TYPE_INT16: return local_kernel_i16(op, p, wide, bytes);
+        case HCCL_DATA_TYPE_UINT16: return local_kernel_u16(op, p, wide, bytes);
+        case HCCL_DATA_TYPE_INT32: return local_kernel_i32(op, p, wide, bytes);
+        case HCCL_DATA_TYPE_UINT32: return local_kernel_u32(op, p, wide, bytes);
+        case HCCL_DATA_TYPE_INT64: return local_kernel_i64(op, p, wide, bytes);
+        case HCCL_DATA_TYPE_UINT64: return local_kernel_u64(op, p, wide, bytes);
+        case HCCL_DATA_TYPE_FP32: return local_kernel_f32(op, p, wide, bytes);
+        case HCCL_DATA_TYPE_FP64: return local_kernel_f64(op, p, wide, bytes);
+        case HCCL_DATA_TYPE_FP16: return local_kernel_f16(op, p, wide, bytes);
+        case HCCL_DATA_TYPE_BFP16: return local_kernel_bf16(op, p, wide, bytes);
         default: return nullptr;
     }
 }
@@ -162,8 +162,8 @@ HcclResult launch_local_copy(LocalCopy &c, void *stream)
 // How a job lies over vectors of vb bytes: outputs first, the sources as they then come.
 static uint32_t layout_of(const LocalReduce &r, LocalReduceJob &j, uint32_t es, uint32_t vb)
 {
+    uint32_t differ = 0, shift = 0;
     const uintptr_t d0 = (uintptr_t)r.out[__builtin_ctz(j.mask)];
-    uint32_t differ = (uint32_t)d0 & (es - 1), shift = 0;  // an output that starts inside an element never meets a vector
     for (uint32_t m = j.mask; m; m &= m - 1) differ |= (uint32_t)((uintptr_t)r.out[__builtin_ctz(m)] ^ d0) & (vb - 1);
     j.head = (uint32_t)std::min<uint64_t>(j.count, ((vb - (d0 & (vb - 1))) & (vb - 1)) / es);
     j.nvec = (j.count - j.head) * es / vb;
@@ -182,12 +182,19 @@ HcclResult launch_local_reduce(LocalReduce &r, int dtype, int redop, void *strea
     if (n == 0) return HCCL_SUCCESS;
     // 32-byte vectors where every address of every job allows them (ReduceScatter of 4 MiB blocks over eight ranks: 43.7 us with
     // them, 46.2 us with 16 bytes), and one width for the whole launch
-    bool wide = true;
+    uintptr_t bits = 0;  // of all addresses, to see whether each is a multiple of the element's size
+    for (int q = 0; q < r.p; ++q) {
+        bits |= (uintptr_t)r.in[q];
+        for (int j = 0; j < n; ++j)
+            if ((r.job[j].mask >> q) & 1u) bits |= (uintptr_t)r.out[q];
+    }
+    const bool bytes = (bits & (es - 1)) != 0;
+    bool wide = !bytes;
     for (int j = 0; j < n && wide; ++j) wide = (r.job[j].layout = layout_of(r, r.job[j], es, 32)) == LOCAL_ALIGNED;
     const uint32_t vb = wide ? 32 : 16;
     uint64_t total = 0;
     for (int j = 0; j < n; ++j) {
-        if (!wide) r.job[j].layout = layout_of(r, r.job[j], es, 16);
+        if (!wide) r.job[j].layout = bytes ? LOCAL_SCALAR : layout_of(r, r.job[j], es, 16);
         total += r.job[j].count * es;
     }
     const uint32_t full = r.p <= 2 ? 64 : (r.p <= 4 ? 32 : vb);  // bytes per thread (kReduceVecs)
@@ -205,7 +212,7 @@ HcclResult launch_local_reduce(LocalReduce &r, int dtype, int redop, void *strea
     }
     r.uniform = uniform ? (uint32_t)same : 0;
     if (tiles > 0x7fffffffu) return HCCL_E_PARA;
-    const void *fn = local_kernel_for(dtype, redop, r.p, wide);
+    const void *fn = local_kernel_for(dtype, redop, r.p, wide, bytes);
     if (!fn) return HCCL_E_PARA;
     return launch_pdl(fn, dim3((unsigned)tiles), kLocalThreads, 0, &r, stream, "direct reduction");
 }

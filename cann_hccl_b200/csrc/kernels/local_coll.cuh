@@ -30,25 +30,6 @@ __device__ __forceinline__ uint4 ld_shifted(const uint8_t *a)
     return s ? merge16(b[0], b[1], s) : b[0];
 }
 
-// One element of a buffer that need not start on a multiple of the element's size: byte by byte where it does not.
-template <class T> union ElemBytes { T e; uint8_t b[sizeof(T)]; __device__ ElemBytes() {} };
-template <class T> __device__ __forceinline__ T ld_elem(const uint8_t *p)
-{
-    if (((uintptr_t)p & (sizeof(T) - 1)) == 0) return *(const T *)p;
-    ElemBytes<T> v;
-#pragma unroll
-    for (int i = 0; i < (int)sizeof(T); ++i) v.b[i] = p[i];
-    return v.e;
-}
-template <class T> __device__ __forceinline__ void st_elem(uint8_t *p, T e)
-{
-    if (((uintptr_t)p & (sizeof(T) - 1)) == 0) { *(T *)p = e; return; }
-    ElemBytes<T> v;
-    v.e = e;
-#pragma unroll
-    for (int i = 0; i < (int)sizeof(T); ++i) p[i] = v.b[i];
-}
-
 // A vector is one load per source: 32 bytes where every address allows it, else 16.
 template <int VB> union Vec;
 template <> union Vec<16> { uint4 u; uint32_t w[4]; };
@@ -140,28 +121,64 @@ __global__ void __launch_bounds__(kLocalThreads) local_reduce_kernel(const __gri
         else if constexpr (VB == 16) local_reduce_tile<T, OP, NP, 16, 1, true>(a, j, tile);
         return;
     }
-    // one by one: what lies outside the vectors (a tile of its own), or everything when the outputs do not share an
-    // alignment or start inside an element
+    // one by one: what lies outside the vectors (a tile of its own), or everything when the outputs do not share an alignment
     const bool scalar = j.layout == LOCAL_SCALAR;
     const uint64_t vecs = scalar ? 0 : j.nvec, left = j.count - vecs * E;
     const uint64_t l0 = scalar ? (uint64_t)tile * a.tile_vecs * E : 0, l1 = scalar ? min(left, l0 + (uint64_t)a.tile_vecs * E) : left;
     for (uint64_t l = l0 + threadIdx.x; l < l1; l += kLocalThreads) {
         const uint64_t e = l < j.head ? l : vecs * E + l;
-        Acc acc = N::up(ld_elem<T>(a.in[0] + j.off + e * sizeof(T)));
-        for (int q = 1; q < a.p; ++q) acc = red_op<OP>(acc, N::up(ld_elem<T>(a.in[q] + j.off + e * sizeof(T))));
+        Acc acc = N::up(((const T *)(a.in[0] + j.off))[e]);
+        for (int q = 1; q < a.p; ++q) acc = red_op<OP>(acc, N::up(((const T *)(a.in[q] + j.off))[e]));
         const T r = N::down(acc);
-        for (uint32_t m = j.mask; m; m &= m - 1) st_elem<T>(a.out[__ffs(m) - 1] + e * sizeof(T), r);
+        for (uint32_t m = j.mask; m; m &= m - 1) ((T *)a.out[__ffs(m) - 1])[e] = r;
     }
 }
 
-// Defines local_kernel_<name>(op, p, wide): the reduction kernel for element type T; wide: vectors of 32 bytes.
+// Some buffer starts inside an element: no vectors, every element byte by byte.  A kernel of its own, because the byte accesses
+// cost the one above registers (bf16, sources merged from aligned vectors: 349 us became 400 us for ReduceScatter of 16 MiB blocks
+// over eight ranks).
+template <class T> union ElemBytes { T e; uint8_t b[sizeof(T)]; __device__ ElemBytes() {} };
+template <class T> __device__ __forceinline__ T ld_bytes(const uint8_t *p)
+{
+    ElemBytes<T> v;
+#pragma unroll
+    for (int i = 0; i < (int)sizeof(T); ++i) v.b[i] = p[i];
+    return v.e;
+}
+template <class T, int OP>
+__global__ void __launch_bounds__(kLocalThreads) local_reduce_bytes_kernel(const __grid_constant__ LocalReduce a)
+{
+    using N = DNum<T>;
+    pdl_trigger();
+    int ji = 0;
+    while (ji + 1 < a.njobs && blockIdx.x >= a.job[ji + 1].tile0) ++ji;
+    const LocalReduceJob &j = a.job[ji];
+    const uint64_t per = (uint64_t)a.tile_vecs * (16 / sizeof(T)), e0 = (uint64_t)(blockIdx.x - j.tile0) * per, e1 = min(j.count, e0 + per);
+    pdl_wait();
+    for (uint64_t e = e0 + threadIdx.x; e < e1; e += kLocalThreads) {
+        const uint64_t b = e * sizeof(T);
+        typename N::Acc acc = N::up(ld_bytes<T>(a.in[0] + j.off + b));
+        for (int q = 1; q < a.p; ++q) acc = red_op<OP>(acc, N::up(ld_bytes<T>(a.in[q] + j.off + b)));
+        ElemBytes<T> r;
+        r.e = N::down(acc);
+        for (uint32_t m = j.mask; m; m &= m - 1) {
+            uint8_t *d = a.out[__ffs(m) - 1] + b;
+#pragma unroll
+            for (int i = 0; i < (int)sizeof(T); ++i) d[i] = r.b[i];
+        }
+    }
+}
+
+// Defines local_kernel_<name>(op, p, wide, bytes): the reduction kernel for element type T; wide: vectors of 32 bytes; bytes: some
+// buffer starts inside an element.
 #define HCCLB_LOCAL_BATCH(T, OP)                                                                                                            \
-    (wide ? (p <= 2 ? (const void *)local_reduce_kernel<T, OP, 2, 32> : p <= 4 ? (const void *)local_reduce_kernel<T, OP, 4, 32>           \
+    (bytes ? (const void *)local_reduce_bytes_kernel<T, OP>                                                                                 \
+     : wide ? (p <= 2 ? (const void *)local_reduce_kernel<T, OP, 2, 32> : p <= 4 ? (const void *)local_reduce_kernel<T, OP, 4, 32>           \
                                                                                : (const void *)local_reduce_kernel<T, OP, 8, 32>)          \
           : (p <= 2 ? (const void *)local_reduce_kernel<T, OP, 2, 16> : p <= 4 ? (const void *)local_reduce_kernel<T, OP, 4, 16>           \
                                                                                : (const void *)local_reduce_kernel<T, OP, 8, 16>))
 #define HCCLB_INSTANTIATE_LOCAL(T, name)                                              \
-    const void *local_kernel_##name(int op, int p, bool wide)                         \
+    const void *local_kernel_##name(int op, int p, bool wide, bool bytes)             \
     {                                                                                 \
         switch (op) {                                                                 \
             case HCCL_REDUCE_SUM: return HCCLB_LOCAL_BATCH(T, HCCL_REDUCE_SUM);       \
