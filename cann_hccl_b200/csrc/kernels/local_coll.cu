@@ -199,12 +199,17 @@ HcclResult launch_local_reduce(LocalReduce &r, int dtype, int redop, void *strea
     }
     const uint32_t full = r.p <= 2 ? 64 : (r.p <= 4 ? 32 : vb);  // bytes per thread (kReduceVecs)
     r.tile_vecs = tile_bytes_for(total, full * kLocalThreads, vb * kLocalThreads) / vb;
+    // one by one: as many elements as the vectors of a tile hold, down to one per thread while that is not two CTAs for every SM
+    // (2 KiB of int8 over eight ranks, outputs of different alignments: 16 elements per thread 17.9 us, one 4.7 us; 1 MiB over two
+    // ranks, 512 CTAs of 16 elements per thread 7.9 us, 2048 CTAs of four 8.9 us)
+    r.tile_elems = r.tile_vecs * (vb / es);
+    while (r.tile_elems > kLocalThreads && total / es / r.tile_elems < 2 * 148) r.tile_elems >>= 1;
     uint64_t tiles = 0, same = 0;
     bool uniform = true;
     for (int j = 0; j < n; ++j) {
         LocalReduceJob &job = r.job[j];
         job.tile0 = (uint32_t)tiles;
-        const uint64_t t = job.layout == LOCAL_SCALAR ? ceil_div_u64(job.count, (uint64_t)r.tile_vecs * (vb / es))
+        const uint64_t t = job.layout == LOCAL_SCALAR ? ceil_div_u64(job.count, r.tile_elems)
                                                       : ceil_div_u64(job.nvec, r.tile_vecs) + (job.nvec * (vb / es) < job.count ? 1 : 0);
         if (j == 0) same = t;
         uniform = uniform && t == same;

@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(kLocalThreads) local_reduce_kernel(const __gri
     // one by one: what lies outside the vectors (a tile of its own), or everything when the outputs do not share an alignment
     const bool scalar = j.layout == LOCAL_SCALAR;
     const uint64_t vecs = scalar ? 0 : j.nvec, left = j.count - vecs * E;
-    const uint64_t l0 = scalar ? (uint64_t)tile * a.tile_vecs * E : 0, l1 = scalar ? min(left, l0 + (uint64_t)a.tile_vecs * E) : left;
+    const uint64_t l0 = scalar ? (uint64_t)tile * a.tile_elems : 0, l1 = scalar ? min(left, l0 + a.tile_elems) : left;
     for (uint64_t l = l0 + threadIdx.x; l < l1; l += kLocalThreads) {
         const uint64_t e = l < j.head ? l : vecs * E + l;
         Acc acc = N::up(((const T *)(a.in[0] + j.off))[e]);
@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(kLocalThreads) local_reduce_bytes_kernel(const
     int ji = 0;
     while (ji + 1 < a.njobs && blockIdx.x >= a.job[ji + 1].tile0) ++ji;
     const LocalReduceJob &j = a.job[ji];
-    const uint64_t per = (uint64_t)a.tile_vecs * (16 / sizeof(T)), e0 = (uint64_t)(blockIdx.x - j.tile0) * per, e1 = min(j.count, e0 + per);
+    const uint64_t e0 = (uint64_t)(blockIdx.x - j.tile0) * a.tile_elems, e1 = min(j.count, e0 + a.tile_elems);
     pdl_wait();
     for (uint64_t e = e0 + threadIdx.x; e < e1; e += kLocalThreads) {
         const uint64_t b = e * sizeof(T);

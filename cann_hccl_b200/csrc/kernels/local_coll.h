@@ -43,7 +43,8 @@ struct LocalReduce {
     uint8_t *out[kMaxRanks];
     LocalReduceJob job[kMaxRanks];
     int p, njobs;
-    uint32_t tile_vecs, uniform;  // uniform: tiles per job when all jobs have the same number, else 0
+    uint32_t tile_vecs, tile_elems;  // of a tile; tile_elems: where a job goes one by one
+    uint32_t uniform;                // tiles per job when all jobs have the same number, else 0
 };
 
 // Both take and change the caller's description (tile tables).

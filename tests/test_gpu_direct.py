@@ -281,3 +281,20 @@ def test_select_names_what_runs(comms):
     one = comms(1)
     one.all_reduce(x[:1], [y[0][:1 << 18]])
     done(one, one.select(L.ALLREDUCE, 1 << 18, L.FP32)[0])
+
+
+@pytest.mark.parametrize("p", [2, 8])
+@pytest.mark.parametrize("dtype", [torch.int8, torch.bfloat16, torch.float64])
+@pytest.mark.parametrize("n", [1, 127, 129, 2048, 37_889, 75_777, 606_209])
+def test_outputs_of_different_alignments(comms, p, dtype, n):
+    """One element after the other: one per thread, a few CTAs more or less than two per SM, and as many as a tile of vectors holds."""
+    c = comms(p)
+    ins = rnd(p, n, dtype, n)
+    base = [torch.full((n + 40,), 9, device="cuda", dtype=dtype) for _ in range(p)]
+    outs = [b[8 + r:8 + r + n] for r, b in enumerate(base)]
+    c.all_reduce(ins, outs, op=L.MAX)
+    done(c)
+    want = reduced(ins, L.MAX)
+    for r, (b, o) in enumerate(zip(base, outs)):
+        assert torch.equal(o.to(want.dtype), want)
+        assert bool((b[:8 + r] == 9).all()) and bool((b[8 + r + n:] == 9).all())
