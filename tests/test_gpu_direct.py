@@ -11,7 +11,8 @@ from cann_hccl_b200 import _lib as L  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 
-# below a vector; around one vector and one tile of 256 threads; around many tiles of the unrolled form
+# below a vector, around one vector, around a few tiles of 128 threads, many tiles (which hold as much as fills a thread's loads in
+# the reductions; the copies' largest tile is test_large_copies)
 SIZES = (1, 3, 17, 4095, 4097, 1_300_001)
 
 
@@ -298,3 +299,58 @@ def test_outputs_of_different_alignments(comms, p, dtype, n):
     for r, (b, o) in enumerate(zip(base, outs)):
         assert torch.equal(o.to(want.dtype), want)
         assert bool((b[:8 + r] == 9).all()) and bool((b[8 + r + n:] == 9).all())
+
+
+@pytest.mark.parametrize("shift", [0, 4, 8, 1])
+def test_large_copies(comms, shift):
+    """More than 20 MB: a thread's full 128 bytes per tile.  Sources at the outputs' alignment, 16 bytes off it, and elsewhere; the
+    size is no multiple of anything."""
+    p, n = 3, 6_100_003
+    c = comms(p)
+    base = [torch.full((n + 40,), float(r), device="cuda") for r in range(p)]
+    base[1].copy_(torch.arange(n + 40, device="cuda") % 16_777_213)
+    bufs = [b[8 + (shift if r == 1 else 0):][:n] for r, b in enumerate(base)]
+    want = bufs[1].clone()
+    c.broadcast(bufs, 1)
+    done(c)
+    for r, (b, x) in enumerate(zip(base, bufs)):
+        assert torch.equal(x, want)
+        if r != 1:
+            assert bool((b[:8] == r).all()) and bool((b[8 + n:] == r).all())
+
+
+@pytest.mark.parametrize("p,root", [(2, 1), (5, 2)])
+def test_rooted_and_variable_in_place(comms, p, root):
+    c = comms(p)
+    n = 50_021
+    big = rnd(p, n * p, torch.float32, 1)
+    want = [big[root][r * n:(r + 1) * n].clone() for r in range(p)]
+    outs = [big[r][r * n:(r + 1) * n] for r in range(p)]
+    c.scatter(big, outs, root)                                   # the root's own block stays where it is
+    done(c)
+    assert all(torch.equal(o, w) for o, w in zip(outs, want))
+    full = rnd(p, n * p, torch.float32, 2)
+    ins = [full[r][r * n:(r + 1) * n] for r in range(p)]
+    want = torch.cat(ins)
+    c.gather(ins, full, root)
+    done(c)
+    assert torch.equal(full[root], want)
+    bufs = rnd(p, n, torch.float32, 3)
+    want = reduced(bufs, L.SUM)
+    c.reduce(bufs, bufs, root)
+    done(c)
+    check(bufs[root], want, torch.float32, p)
+    counts = np.array([1000 + 37 * r for r in range(p)], np.uint64)
+    displs = np.array([5 + 1500 * r for r in range(p)], np.uint64)
+    cut = lambda x, r: x[int(displs[r]):int(displs[r] + counts[r])]
+    full = rnd(p, n, torch.float32, 4)
+    want = [cut(full[r], r).clone() for r in range(p)]
+    c.all_gather_v([cut(full[r], r) for r in range(p)], full, counts, displs)
+    done(c)
+    assert all(torch.equal(cut(f, r), want[r]) for f in full for r in range(p))
+    ins = rnd(p, n, torch.float32, 5)
+    want = reduced(ins, L.SUM)
+    c.reduce_scatter_v(ins, [cut(ins[r], r) for r in range(p)], counts, displs)
+    done(c)
+    for r in range(p):
+        check(cut(ins[r], r), cut(want, r), torch.float32, p)
