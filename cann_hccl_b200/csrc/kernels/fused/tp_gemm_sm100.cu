@@ -40,6 +40,7 @@
 #include "common/log.h"
 #include "core/device_api.h"
 #include "kernels/fused/tc05.cuh"
+#include "kernels/fused/tensor_map.h"
 #include "kernels/fused/tp_gemm.h"
 #include "kernels/fused/tp_gemm_noalloc.h"
 #include "kernels/prims.cuh"
@@ -608,24 +609,6 @@ __global__ void __launch_bounds__(kThreads, 1) tp_gemm_pair_kernel(const __grid_
     extern __shared__ uint8_t smem_raw[];
     SharedStorage &S = *(SharedStorage *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     tp_gemm_body<true>(PA.r[blockIdx.y], S);
-}
-
-HcclResult encode_2d(CUtensorMap *map, const void *base, uint64_t rows, uint64_t cols, uint32_t box_rows)
-{
-    const DriverApi &d = driver_api();
-    if (!d.ok || !d.TensorMapEncodeTiled) return HCCL_E_DRV;
-    cuuint64_t dims[2] = {cols, rows};
-    cuuint64_t strides[1] = {cols * 2};
-    cuuint32_t box[2] = {(cuuint32_t)BK, box_rows};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = d.TensorMapEncodeTiled(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box, estr,
-                                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-        HLOG_ERROR("cuTensorMapEncodeTiled failed: %s", cu_err(r));
-        return HCCL_E_DRV;
-    }
-    return HCCL_SUCCESS;
 }
 
 }  // namespace
