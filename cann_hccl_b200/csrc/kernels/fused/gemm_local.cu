@@ -399,10 +399,11 @@ int shard_tiles(const GemmCall &c, int cols) { return (c.N + cols - 1) / cols; }
 // Estimated time (ns) of a tiling: the slowest unit (its rows of A and B per k step, which L2 delivers at 128 bytes per 0.8 to
 // 1 ns, and the epilogues), against what the power cap leaves the tensor cores (a narrower tile reads more shared memory per
 // product; of a wave that is partly idle about a quarter shows, the clock takes back the rest) and what HBM delivers.  The
-// constants are a fit to 1200 (shape, tiling) pairs, 128 to 2048 rows, 1024 to 28672 columns and depth: the chosen tiling was
-// within 3 % of the best one measured for each of the 21 shapes.  256 columns everywhere lost up to a third: 128 x 4096 x 1024
-// 10.3 us, with 64 columns 6.6; 640 x 4096 x 11008 65 us, with 144 columns 47; 128 x 28672 x 8192 84 us, with 208 columns 78;
-// 2048 x 8192 x 28672 696 us, with 224 columns (four whole waves) 665.
+// constants are a fit to measured (shape, tiling) pairs, 128 to 2048 rows, 1024 to 28672 columns and depth; over 21 such shapes the
+// chosen tiling is within 5 % of the best one measured (20 of them within 3 %).  256 columns everywhere lose up to a factor of
+// three: 128 x 4096 x 1024 10.7 us, with 64 columns 7.1; 640 x 4096 x 11008 71 us, with 144 columns 48; 128 x 28672 x 8192 83 us,
+// with 208 columns 79; 2048 x 8192 x 28672 656 us, with 224 columns (four whole waves) 619; 128 x 2560 x 8192 51 us, with 80 columns
+// split in four 15.
 double tiling_ns(const GemmCall &c, const Tiling &t, int units)
 {
     const int k_iters = c.K / BK * (c.form == GEMM_REDUCE ? c.p : 1);

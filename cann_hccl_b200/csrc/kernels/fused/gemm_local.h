@@ -23,7 +23,7 @@ struct GemmCall {
 };
 // status: host-mapped block that records a wait that ran out (may be null).
 HcclResult launch_gemm_local(const GemmCall &c, DevStatus *status, void *stream);
-// Launches so far: 128 x 256 tiles of single CTAs, 256 x 256 tiles of two CTAs.
+// Launches so far: tiles of 128 rows on single CTAs, tiles of 256 rows on pairs (64 to 256 columns either way).
 void gemm_local_launch_counts(uint64_t *single, uint64_t *pair);
 
 }  // namespace hcclb

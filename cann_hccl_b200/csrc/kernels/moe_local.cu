@@ -11,10 +11,11 @@
 // Up to 65536 pairs over all ranks, the rows come from ONE cluster that counts in shared memory and registers.
 //
 // Bound: HBM for prefill batches (8192 tokens x 7168, top 8, one rank: dispatch 165 us at 6.4 TB/s, combine 156 us at 6.8 TB/s,
-// whole exchange 337 us, 468 us with a row read per expert, a launch per rank and step, and barriers), launches and L2 for
-// decode batches (128 tokens on each of four ranks: 25 us, 301 us before).  Dispatch with 16-byte instead of 32-byte vectors:
-// 171 us.  Rows of 7224 pairs: 1 CTA 16.3 us for the whole exchange (903 tokens x 1280), four CTAs 15.1 us; 65536 pairs counted
-// through global memory: 340 us, by the cluster 338 us.  Combine of 6516 tokens x 3840, top 4, with one token per CTA: 51 us, with
+// whole exchange 338 us, 468 us with a row read per expert, a launch per rank and step, and barriers), launches and L2 for
+// decode batches (128 tokens on each of four ranks: 25.9 us, 294 us before; 25.4 us with activations and experts loaded ahead of
+// the dispatch's own wait, which is not sound).  Dispatch with 16-byte instead of 32-byte vectors: 171 us.  Whole exchange,
+// rows of 7224 pairs (903 tokens x 1280): 1 CTA 15.1 us, four CTAs 13.6 us, through global memory 16.1 us; of 26064 pairs (6516
+// tokens x 3840, top 4) by the cluster 91.9 us, through global memory 94.0 us; of 65536 pairs 338 and 337 us.  Combine of 6516 tokens x 3840, top 4, with one token per CTA: 51 us, with
 // two 45 us; 32-byte instead of 16-byte loads cost occupancy (8192 x 7168, top 8: 159 -> 171 us).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
