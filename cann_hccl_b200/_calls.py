@@ -29,7 +29,7 @@ class Calls:
 
     def op(self, comm, nlocal, coll, algo, nchan, op, root, send, recv, stream, by_recv, divide):
         of = recv if by_recv else send
-        if isinstance(of, (list, tuple)) and of:
+        if nlocal > 1 or (isinstance(of, (list, tuple)) and of):
             of = of[0]
         if stream is None:
             stream = self._get_stream(self._get_device())

@@ -115,11 +115,9 @@ static int stream_of(PyObject *x, void **out)
     return *out == NULL && PyErr_Occurred() ? -1 : 0;
 }
 
-/* elements and HcclDataType of a tensor or numpy array (the first one of a list) */
-static int describe(PyObject *x, uint64_t *count, int32_t *dtype)
+/* elements and HcclDataType of a tensor or numpy array */
+static int describe_one(PyObject *x, uint64_t *count, int32_t *dtype)
 {
-    if (PyList_Check(x) && PyList_GET_SIZE(x)) x = PyList_GET_ITEM(x, 0);
-    else if (PyTuple_Check(x) && PyTuple_GET_SIZE(x)) x = PyTuple_GET_ITEM(x, 0);
     PyObject *n = PyObject_CallMethodNoArgs(x, s_numel);
     if (!n) {
         if (!PyErr_ExceptionMatches(PyExc_AttributeError)) return -1;
@@ -142,6 +140,18 @@ static int describe(PyObject *x, uint64_t *count, int32_t *dtype)
     return PyErr_Occurred() ? -1 : 0;
 }
 
+/* of the first buffer of a list, a tuple or, where there are several ranks, any other sequence */
+static int describe(PyObject *x, Py_ssize_t nlocal, uint64_t *count, int32_t *dtype)
+{
+    const int list = PyList_Check(x) || PyTuple_Check(x);
+    if ((!list && nlocal == 1) || (list && PySequence_Fast_GET_SIZE(x) == 0)) return describe_one(x, count, dtype);
+    PyObject *first = PySequence_GetItem(x, 0);
+    if (!first) return -1;
+    const int rc = describe_one(first, count, dtype);
+    Py_DECREF(first);
+    return rc;
+}
+
 /* op(comm, nlocal, coll, algo, nchan, op, root, send, recv, stream, by_recv, divide) -> result code: a collective whose count and
  * type are those of the send buffer (by_recv: of the receive buffer), the count divided by `divide` */
 static PyObject *op(PyObject *self, PyObject *const *a, Py_ssize_t n)
@@ -156,7 +166,7 @@ static PyObject *op(PyObject *self, PyObject *const *a, Py_ssize_t n)
     const uint64_t divide = PyLong_AsUnsignedLongLong(a[11]);
     if (PyErr_Occurred()) return NULL;
     if (nlocal < 1 || nlocal > MAX_LOCAL || !divide) { PyErr_SetString(PyExc_ValueError, "bad number of local ranks"); return NULL; }
-    if (describe(a[10] == Py_True ? a[8] : a[7], &o.count, &o.dataType)) return NULL;
+    if (describe(a[10] == Py_True ? a[8] : a[7], nlocal, &o.count, &o.dataType)) return NULL;
     o.count /= divide;
     void *send[MAX_LOCAL], *recv[MAX_LOCAL];
     if (addresses(a[7], nlocal, send) || addresses(a[8], nlocal, recv) || stream_of(a[9], &stream)) return NULL;

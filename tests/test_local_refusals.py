@@ -201,6 +201,13 @@ def test_buffers_as_rows_of_one_array(pair):
     tx, ty = torch.arange(10.).reshape(2, 5), torch.zeros(2, 5)
     pair.collective(L.ALLREDUCE, tx, ty, 5, L.FP32)
     assert torch.equal(ty, tx.sum(0).repeat(2, 1))
+    for call, count in (("all_reduce", 5), ("all_gather", 5), ("reduce_scatter", 4), ("all_to_all", 4)):  # a row's count, not the array's
+        src = np.arange(16, dtype=np.float32).reshape(2, 8)[:, :count if call != "reduce_scatter" else 8].copy()
+        dst = np.full((2, 16), -1, np.float32)[:, :{"all_reduce": 5, "all_gather": 10, "reduce_scatter": 4, "all_to_all": 4}[call]].copy()
+        lists = [d.copy() for d in dst]
+        getattr(pair, call)(src, dst)
+        getattr(pair, call)(list(src), lists)
+        assert np.array_equal(dst, np.stack(lists)) and (dst >= 0).all()
     for bad in (x[:1], [x[0]], (x[0], x[0], x[1])):
         with pytest.raises(AssertionError):
             pair.collective(L.ALLREDUCE, bad, y, 5, L.FP32)
