@@ -622,6 +622,11 @@ static bool null_buffer(const OpRequest &rq, int p, int rank, int li)
     op_byte_ranges(rq, p, rank, &ib, &ob);
     if (rq.coll == COLL_ALLTOALLV || rq.coll == COLL_ALLTOALLVC)
         for (int j = 0; j < p; ++j) { ib |= rq.send_counts[(size_t)li * p + j]; ob |= rq.recv_counts[(size_t)li * p + j]; }
+    if (rq.coll == COLL_ALLGATHER_V || rq.coll == COLL_REDUCE_SCATTER_V) {
+        uint64_t any = 0;  // displacements alone touch nothing
+        for (int j = 0; j < p; ++j) any |= rq.counts[j];
+        if (!any) return false;
+    }
     return (ib && !(rq.in && rq.in[li])) || (ob && !(rq.out && rq.out[li]));
 }
 

@@ -180,6 +180,9 @@ def test_collectives_with_a_null_buffer(pair):
     out = [np.zeros(n, np.float32), None]                       # only the root receives
     pair.reduce(x, out, 0)
     assert np.array_equal(out[0], 2 * x[0])
+    zero, at = np.zeros(2, np.uint64), np.array([3, 5], np.uint64)
+    pair.collective(L.ALLGATHER_V, [None, None], [None, None], 0, L.FP32, counts=zero, displs=at)
+    pair.collective(L.REDUCE_SCATTER_V, [None, None], [None, None], 0, L.FP32, counts=zero, displs=at)
     c = np.array([[0, 2], [0, 0]], np.uint64)
     d = np.zeros((2, 2), np.uint64)
     got = [None, np.zeros(2, np.float32)]                       # rank 0 only sends, rank 1 only receives
